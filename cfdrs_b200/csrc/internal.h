@@ -311,8 +311,9 @@ struct cfd_context {
   int* err = nullptr;    // set by a kernel whose bounded wait ran out
   int* h_err = nullptr;  // pinned mirror
   int num_sms = 148;
-  // CG / Jacobi-PCG of small systems as one thread-block-cluster launch
-  // (cluster_pcg.cu) where the system fits; cfd_context_set_cluster_solve
+  // CG / Jacobi-PCG (cluster_pcg.cu) and FP64 GMRES (cluster_gmres.cu) of small
+  // systems as one thread-block-cluster launch where the system fits;
+  // cfd_context_set_cluster_solve
   bool cluster_solve = true;
   cfd::KernelStats stats;
   std::mutex mu;
@@ -361,4 +362,8 @@ cfd_status pattern_outer_launch(cfd_csr* a, const double* lambda, const double* 
 // *ok = false (nothing launched) when the system does not fit.
 cfd_status cluster_pcg_solve(cfd_context* ctx, const DevMat& m, const double* jinv, const double* b, double* x,
                              DevState* st, bool* ok);
+// Whole GMRES(m) solve (no preconditioner, Jacobi or AMG) in one thread-block
+// cluster (cluster_gmres.cu): *ok = false (nothing launched) when it does not fit.
+cfd_status cluster_gmres_solve(cfd_context* ctx, const cfd_csr* a, cfd_amg* amg, int precond, int m, const double* b,
+                               double* x, DevState* st, DevState* host_st, bool* ok);
 }  // namespace cfd

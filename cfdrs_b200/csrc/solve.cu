@@ -1332,18 +1332,7 @@ cfd_status solve_fp64(cfd_csr* a, const cfd_solve_options& opt, cfd_amg* amg, co
   const bool host_mem = opt.memory == CFD_MEMORY_HOST;
   B.x = host_mem ? al.get(n) : x;
   B.b = host_mem ? al.get(n) : const_cast<double*>(b);
-  B.r = al.get(n);
-  B.p = al.get(n);
-  B.q = al.get(n);
-  B.z = al.get(n);
-  if (opt.solver == CFD_SOLVER_BICGSTAB) {
-    B.rh = al.get(n);
-    B.v = al.get(n);
-    B.s = al.get(n);
-    B.sh = al.get(n);
-    B.t = al.get(n);
-  }
-  if (!B.x || !B.b || !B.r || !B.p || !B.q || !B.z || (opt.solver == CFD_SOLVER_BICGSTAB && !B.t)) {
+  if (!B.x || !B.b) {
     set_error("device workspace allocation failed (%lld unknowns)", (long long)n);
     return CFD_ERR_ALLOC;
   }
@@ -1356,18 +1345,35 @@ cfd_status solve_fp64(cfd_csr* a, const cfd_solve_options& opt, cfd_amg* amg, co
     CFD_TRY_CUDA(cudaMemcpyAsync(B.x, x, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   }
   CFD_TRY_CUDA(cudaMemcpyAsync(st, hs, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));
-  if (opt.solver == CFD_SOLVER_BICGSTAB) {
-    CFD_TRY_CUDA(cudaMemsetAsync(B.v, 0, n * sizeof(double), ctx->stream));
-    CFD_TRY_CUDA(cudaMemsetAsync(B.p, 0, n * sizeof(double), ctx->stream));
-  }
   Poller pl{ctx, st, hs};
   pl.fixed = opt.check_every;
+  const bool plain_pre = opt.precond == CFD_PRECOND_NONE || opt.precond == CFD_PRECOND_JACOBI;
   bool whole = false;
-  if (ctx->cluster_solve && opt.solver == CFD_SOLVER_CG &&
-      (opt.precond == CFD_PRECOND_NONE || opt.precond == CFD_PRECOND_JACOBI))
+  if (ctx->cluster_solve && opt.solver == CFD_SOLVER_CG && plain_pre)
     CFD_TRY(cluster_pcg_solve(ctx, a->dev, opt.precond == CFD_PRECOND_JACOBI ? a->jinv64 : nullptr, B.b, B.x, st,
                               &whole));
+  if (ctx->cluster_solve && opt.solver == CFD_SOLVER_GMRES && (plain_pre || opt.precond == CFD_PRECOND_AMG))
+    CFD_TRY(cluster_gmres_solve(ctx, a, amg, opt.precond, gmres_width(opt.restart), B.b, B.x, st, hs, &whole));
   if (!whole) {
+    B.r = al.get(n);
+    B.p = al.get(n);
+    B.q = al.get(n);
+    B.z = al.get(n);
+    if (opt.solver == CFD_SOLVER_BICGSTAB) {
+      B.rh = al.get(n);
+      B.v = al.get(n);
+      B.s = al.get(n);
+      B.sh = al.get(n);
+      B.t = al.get(n);
+    }
+    if (!B.r || !B.p || !B.q || !B.z || (opt.solver == CFD_SOLVER_BICGSTAB && !B.t)) {
+      set_error("device workspace allocation failed (%lld unknowns)", (long long)n);
+      return CFD_ERR_ALLOC;
+    }
+    if (opt.solver == CFD_SOLVER_BICGSTAB) {
+      CFD_TRY_CUDA(cudaMemsetAsync(B.v, 0, n * sizeof(double), ctx->stream));
+      CFD_TRY_CUDA(cudaMemsetAsync(B.p, 0, n * sizeof(double), ctx->stream));
+    }
     // r0 = b - A x0, ||r0||, threshold, InitialResidual test.
     CFD_TRY(lc.spmv<double, double, false>(a->dev, B.x, EpiResidual<double, 1>{B.r, B.b, st, nullptr, {}}));
     CFD_TRY(krylov_loop<double>(lc, opt.solver, opt.precond, a, amg, B, st, pl, opt.restart));
