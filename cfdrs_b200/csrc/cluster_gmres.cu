@@ -175,7 +175,6 @@ struct GcCta {
   uint32_t base;  // shared address of sm
   int rank, ncta;
   __device__ double* d(int off) const { return reinterpret_cast<double*>(sm + off); }
-  __device__ const uint16_t* u(int off) const { return reinterpret_cast<const uint16_t*>(sm + off); }
 };
 
 __device__ __forceinline__ int gc_rows(int n, int rpc, int rank) { return max(0, min(rpc, n - rank * rpc)); }

@@ -6,17 +6,31 @@
 //
 // A multi-kernel PCG iteration on such a system is bound by launch and
 // grid-reduction latency (about 19 us per iteration at 128^2: three to four
-// kernels on data that sits in L2). Here one launch runs the whole solve:
-// every CTA of the cluster keeps its block of rows (CSR values, columns as
-// (owning CTA, local index), row offsets) and its slices of x, r, p, q and
-// D^-1 in shared memory; the SpMV reads p of other rows from their owners'
-// shared memory (distributed shared memory); a dot product is a per-CTA partial
-// written to shared memory, one cluster barrier, and every CTA summing all
-// partials in rank order, so every CTA holds the same value and takes the same
-// branch. Three cluster barriers per iteration: before the SpMV (p complete),
-// after the p.q partials, after the r.r and r.z partials. The barriers are the
-// hardware cluster barrier; control flow is uniform across the cluster, so no
-// CTA can wait for one that has left.
+// kernels on data that sits in L2). Here one launch runs the whole solve, and an
+// iteration is bound by two cluster barriers (450 cycles each with release and
+// acquire), one remote gather (325 cycles) and the two reductions' shuffles:
+//  - A thread owns R rows: x, r, p, q and D^-1 of those rows, and up to two
+//    rows a thread the first entries of the matrix, stay in registers; z = D^-1 r
+//    and p are also in shared memory, where the other rows read them.
+//  - The SpMV forms another CTA's new direction itself, z_j + beta p_j from that
+//    CTA's z and old p (two buffers of p in turn), so p needs no barrier of its
+//    own; the same operations as the owner's, so the same bits. Only lanes whose
+//    entry is another CTA's take the cluster path (a predicate on the load): its
+//    throughput is low even for a CTA's own memory (SpMV phase 1600 -> 1190
+//    cycles at 128^2).
+//  - A row's five entries are read without branches (slots past its end take a
+//    zero entry), so all of its gathers are in flight together.
+//  - Behind a reduction's barrier one warp fetches the CTAs' partials (one
+//    remote load) and hands the totals to the others; pushing them to every CTA
+//    before the barrier made the barrier wait for the stores (3.65 against 3.08
+//    us an iteration).
+// Every CTA sums all partials in the same order, so every CTA holds the same
+// value and takes the same branch. The barriers are the hardware cluster
+// barrier; control flow is uniform across the cluster, so no CTA can wait for
+// one that has left. Measured, Jacobi-CG to 1e-10, device time before (three
+// barriers an iteration, vectors in shared memory, entry-by-entry gathers of p)
+// and now: 64^2 0.99 -> 0.53 ms, 128^2 2.03 -> 1.30 ms, 181^2 3.74 -> 2.43 ms,
+// 200 x 170 4.92 -> 2.96 ms.
 //
 // Recurrence and termination are pcg_loop's: r0 = b - A x0, threshold
 // max(tol, rtol ||r0||), InitialResidual / Breakdown on the initial residual;
@@ -32,7 +46,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <vector>
 
 #include "internal.h"
 #include "kernels.cuh"
@@ -43,7 +56,10 @@ namespace cfd {
 namespace {
 
 constexpr int kClThreads = 512;
+constexpr int kClWarps = kClThreads / 32;
 constexpr int kClMaxCtas = 16;
+constexpr int kClMaxRows = 8;  // rows per thread
+constexpr int kClU = 5;        // entries of a row read together (a five-point row)
 
 struct ClusterArgs {
   const int* __restrict__ rp;  // global CSR (int32)
@@ -57,44 +73,47 @@ struct ClusterArgs {
 };
 
 struct ClusterLayout {
-  size_t val, ent, rpl, vec, bytes;
+  size_t val, ent, rpl, z, p, bytes;
 };
 
 __host__ __device__ inline size_t cl_round16(size_t b) { return (b + 15) / 16 * 16; }
 
 __host__ __device__ inline ClusterLayout cluster_layout(int rpc, int nnz_cap) {
   ClusterLayout L;
-  L.val = 0;
-  L.ent = cl_round16((size_t)nnz_cap * 8);
-  L.rpl = L.ent + cl_round16((size_t)nnz_cap * 4);
-  L.vec = L.rpl + cl_round16((size_t)(rpc + 1) * 4);
-  L.bytes = L.vec + 5 * cl_round16((size_t)rpc * 8);
+  L.val = 0;  // nnz_cap values and a zero entry
+  L.ent = cl_round16((size_t)(nnz_cap + 1) * 8);
+  L.rpl = L.ent + cl_round16((size_t)(nnz_cap + 1) * 4);
+  L.z = L.rpl + cl_round16((size_t)(rpc + 1) * 4);
+  L.p = L.z + cl_round16((size_t)rpc * 8);
+  L.bytes = L.p + 2 * cl_round16((size_t)rpc * 8);  // two buffers
   return L;
 }
 
-// Sums of a and b over the CTA, written by thread 0 to out[0..1].
-__device__ __forceinline__ void cl_block_sum2(double a, double b, double (&buf)[2][32], double* out) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  a = warp_sum(a);
-  b = warp_sum(b);
-  if (lane == 0) {
-    buf[0][w] = a;
-    buf[1][w] = b;
-  }
-  __syncthreads();
-  if (w == 0) {
-    const int nw = (int)(blockDim.x >> 5);
-    double ta = lane < nw ? buf[0][lane] : 0.0, tb = lane < nw ? buf[1][lane] : 0.0;
-    ta = warp_sum(ta);
-    tb = warp_sum(tb);
-    if (lane == 0) {
-      out[0] = ta;
-      out[1] = tb;
-    }
-  }
+__device__ __forceinline__ uint32_t cl_map(uint32_t a, uint32_t rank) {
+  uint32_t d;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(rank));
+  return d;
+}
+// Loads and stores of the cluster's shared memory. Volatile keeps them between
+// the barriers that order them; consecutive loads still overlap.
+// The load only where `on` (a predicate, not a branch), else v as it is: the
+// cluster path is slow even for a CTA's own memory, so only lanes whose entry is
+// another CTA's take it.
+__device__ __forceinline__ void cl_ld_if(double& v, uint32_t a, bool on) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q ld.shared::cluster.f64 %0, [%1];\n}\n"
+               : "+d"(v)
+               : "r"(a), "r"((int)on));
+}
+__device__ __forceinline__ void cl_st(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cl_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(kClThreads) k_cluster_pcg(ClusterArgs A) {
+template <int R>
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int ncta = (int)cluster.num_blocks();
@@ -103,105 +122,231 @@ __global__ void __launch_bounds__(kClThreads) k_cluster_pcg(ClusterArgs A) {
   double* sval = reinterpret_cast<double*>(sm + L.val);
   int* sent = reinterpret_cast<int*>(sm + L.ent);  // owner << 16 | local index
   int* srp = reinterpret_cast<int*>(sm + L.rpl);
-  const size_t vs = cl_round16((size_t)A.rpc * 8);
-  double* sx = reinterpret_cast<double*>(sm + L.vec);
-  double* sr = reinterpret_cast<double*>(sm + L.vec + vs);
-  double* sp = reinterpret_cast<double*>(sm + L.vec + 2 * vs);
-  double* sq = reinterpret_cast<double*>(sm + L.vec + 3 * vs);
-  double* sj = reinterpret_cast<double*>(sm + L.vec + 4 * vs);
+  double* sz = reinterpret_cast<double*>(sm + L.z);
+  const uint32_t psz = (uint32_t)cl_round16((size_t)A.rpc * 8);  // bytes of a p buffer
+  auto sp = [&](int buf) { return reinterpret_cast<double*>(sm + L.p + (buf ? psz : 0u)); };
   __shared__ double part[2][2];  // [slot][value]: this CTA's partial sums
-  __shared__ double redbuf[2][32];
-  __shared__ double tot[2];
-  __shared__ double* px[kClMaxCtas];  // every CTA's x and p in the cluster's shared window
-  __shared__ double* pp[kClMaxCtas];
+  __shared__ double bcast[2];
+  __shared__ double red[2][kClWarps];
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+  const uint32_t pbase = (uint32_t)__cvta_generic_to_shared(&part[0][0]);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   const int r0 = rank * A.rpc;
   const int nrow = max(0, min(A.rpc, A.n - r0));
   const int k0 = nrow > 0 ? A.rp[r0] : 0;
   const int nnz = nrow > 0 ? A.rp[r0 + nrow] - k0 : 0;
-  for (int i = threadIdx.x; i <= nrow; i += blockDim.x) srp[i] = A.rp[r0 + i] - k0;
-  for (int e = threadIdx.x; e < nnz; e += blockDim.x) {
+  for (int i = tid; i <= nrow; i += kClThreads) srp[i] = nrow > 0 ? A.rp[r0 + i] - k0 : 0;
+  for (int e = tid; e < nnz; e += kClThreads) {
     const int c = A.col[k0 + e];
     const int owner = c / A.rpc;
     sent[e] = (owner << 16) | (c - owner * A.rpc);
     sval[e] = A.val[k0 + e];
   }
-  for (int i = threadIdx.x; i < nrow; i += blockDim.x) {
-    sx[i] = A.x[r0 + i];
-    sj[i] = A.jinv ? A.jinv[r0 + i] : 1.0;
+  if (tid == 0) {  // the zero entry: this CTA's first vector entry times 0
+    sent[A.nnz_cap] = rank << 16;
+    sval[A.nnz_cap] = 0.0;
   }
-  if (threadIdx.x < ncta) {
-    px[threadIdx.x] = cluster.map_shared_rank(sx, threadIdx.x);
-    pp[threadIdx.x] = cluster.map_shared_rank(sp, threadIdx.x);
-  }
-  cluster.sync();  // every CTA's x staged
-
-  auto row_sum = [&](int i, double* const* vec) {
-    double s = 0.0;
-    for (int k = srp[i]; k < srp[i + 1]; ++k) {
-      const int e = sent[k];
-      s += sval[k] * vec[e >> 16][e & 0xffff];
+  double x[R], r[R], p[R], q[R], jv[R];
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    const int i = tid + u * kClThreads;
+    const bool live = i < nrow;
+    x[u] = live ? A.x[r0 + i] : 0.0;
+    jv[u] = live ? (A.jinv ? A.jinv[r0 + i] : 1.0) : 0.0;
+    r[u] = p[u] = q[u] = 0.0;
+    if (i < A.rpc) {
+      sz[i] = x[u];
+      sp(0)[i] = 0.0;
+      sp(1)[i] = x[u];
     }
-    return s;
+  }
+  cl_barrier();  // every CTA's x staged (in z and the second p buffer)
+
+  // Up to two rows a thread keep their first kClU entries in registers: read
+  // from shared memory every iteration they bound the SpMV (12 of 20 bytes an
+  // entry at 128 bytes a cycle).
+  constexpr bool kKeep = R <= 2;
+  // rows side by side, so that their gathers overlap, where the registers allow it
+  constexpr int G = R == 2 || R == 4 ? 2 : 1;
+  struct Entries {
+    int c[kClU];
+    double v[kClU];
   };
-  // CTA partials -> cluster totals: lane k of warp 0 fetches CTA k's partials
-  // and the warp sums them by a fixed butterfly, so every CTA gets the same bits
-  auto cluster_totals = [&](int slot, double a, double b2, double* ta, double* tb) {
-    cl_block_sum2(a, b2, redbuf, &part[slot][0]);
-    cluster.sync();
-    if (threadIdx.x < 32) {
-      const int lane = threadIdx.x;
-      double ua = 0.0, ub = 0.0;
-      if (lane < ncta) {
-        const double* pk = cluster.map_shared_rank(&part[slot][0], lane);
-        ua = pk[0];
-        ub = pk[1];
+  auto entries = [&](Entries& E, int k, int ke) {
+#pragma unroll
+    for (int w = 0; w < kClU; ++w) {
+      const int e = k + w < ke ? k + w : A.nnz_cap;
+      E.c[w] = sent[e];
+      E.v[w] = sval[e];
+    }
+  };
+  auto bounds = [&](int u, int& k, int& ke) {
+    const int i = min(tid + u * kClThreads, nrow);  // row nrow: empty
+    k = srp[i];
+    ke = srp[min(i + 1, nrow)];
+  };
+  Entries kept[kKeep ? R : 1];
+  int kbeg[kKeep ? R : 1], kend[kKeep ? R : 1];
+  if constexpr (kKeep) {
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      bounds(u, kbeg[u], kend[u]);
+      entries(kept[u], kbeg[u], kend[u]);
+    }
+  }
+  // sum_j a_ij p_j over the thread's rows, p the new direction: this CTA's own
+  // from its p buffer (complete in the CTA), another CTA's formed here from
+  // that CTA's z and old p
+  auto row_sums = [&](int buf, double beta, double (&out)[R]) {
+    const uint32_t zb = base + (uint32_t)L.z;
+    const uint32_t dold = (uint32_t)(L.p - L.z) + (buf ? psz : 0u);
+    const double* pn = sp(buf ^ 1);
+#pragma unroll
+    for (int u0 = 0; u0 < R; u0 += G) {
+      Entries E[G];
+      int k[G], ke[G];
+      double s[G];
+      bool more = false;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        if constexpr (kKeep) {
+          E[g] = kept[u0 + g];
+          k[g] = kbeg[u0 + g];
+          ke[g] = kend[u0 + g];
+        } else {
+          bounds(u0 + g, k[g], ke[g]);
+          entries(E[g], k[g], ke[g]);
+        }
+        s[g] = 0.0;
+        more |= k[g] < ke[g];
       }
-      ua = warp_sum(ua);
-      ub = warp_sum(ub);
-      if (lane == 0) {
-        tot[0] = ua;
-        tot[1] = ub;
+      while (more) {
+        bool own = true;
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+          for (int w = 0; w < kClU; ++w) own &= (E[g].c[w] >> 16) == rank;
+        double x[G][kClU];
+        if (__all_sync(__activemask(), own)) {
+#pragma unroll
+          for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int w = 0; w < kClU; ++w) x[g][w] = pn[E[g].c[w] & 0xffff];
+        } else {
+          double pv[G][kClU];
+#pragma unroll
+          for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int w = 0; w < kClU; ++w) {
+              const int c = E[g].c[w], owner = c >> 16;
+              const bool far = owner != rank;
+              const uint32_t at = cl_map(zb + 8u * (uint32_t)(c & 0xffff), (uint32_t)owner);
+              x[g][w] = pn[far ? 0 : c & 0xffff];
+              pv[g][w] = 0.0;
+              cl_ld_if(x[g][w], at, far);
+              cl_ld_if(pv[g][w], at + dold, far);
+            }
+#pragma unroll
+          for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int w = 0; w < kClU; ++w) x[g][w] = fma(beta, pv[g][w], x[g][w]);
+        }
+        more = false;
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+#pragma unroll
+          for (int w = 0; w < kClU; ++w) s[g] = fma(E[g].v[w], x[g][w], s[g]);
+          k[g] += kClU;
+          more |= k[g] < ke[g];
+        }
+        if (more) {
+#pragma unroll
+          for (int g = 0; g < G; ++g) entries(E[g], k[g], ke[g]);
+        }
       }
+#pragma unroll
+      for (int g = 0; g < G; ++g) out[u0 + g] = s[g];
+    }
+  };
+  // CTA partials pushed to every CTA, one barrier, then summed in rank order:
+  // every CTA gets the same bits. Two slots in turn: a CTA pushes into a slot
+  // again only after a barrier that the others pass behind their reads of it.
+  int slot = 0;
+  auto totals = [&](double a, double b2, double& ta, double& tb) {
+    // both sums folded at once: the lower half-warp takes a, the upper b2
+    const bool up = lane >= 16;
+    auto fold = [&](double t) {
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      return t;
+    };
+    const double got = __shfl_xor_sync(0xffffffffu, up ? a : b2, 16);
+    double t = fold((up ? b2 : a) + got);
+    if ((lane & 15) == 0) red[up][warp] = t;
+    __syncthreads();
+    if (warp == 0) {
+      t = fold(red[up][lane & 15]);
+      if ((lane & 15) == 0) part[slot][up] = t;
+    }
+    cl_barrier();
+    if (warp == 0) {
+      t = 0.0;
+      cl_ld_if(t, cl_map(pbase + (uint32_t)(slot * 2 + up) * 8u, (uint32_t)(lane & 15)), (lane & 15) < ncta);
+      t = fold(t);
+      if ((lane & 15) == 0) bcast[up] = t;
     }
     __syncthreads();
-    *ta = tot[0];
-    *tb = tot[1];
-    __syncthreads();  // tot is rewritten by the next reduction
+    ta = bcast[0];
+    tb = bcast[1];
+    slot ^= 1;
   };
+  static_assert(kClWarps == 16 && kClMaxCtas == 16, "the folds take 16 partials");
 
-  // r0 = b - A x0, z0 = D^-1 r0, p0 = z0, rho = r0.z0
+  // r0 = b - A x0, z0 = D^-1 r0, rho = r0.z0 (x was staged in z and the
+  // second p buffer, the old p in the first is zero)
   double arr = 0.0, arz = 0.0;
-  for (int i = threadIdx.x; i < nrow; i += blockDim.x) {
-    const double ri = A.b[r0 + i] - row_sum(i, px);
-    sr[i] = ri;
-    const double zi = ri * sj[i];
-    sp[i] = zi;
-    arr += ri * ri;
-    arz += ri * zi;
+  row_sums(0, 0.0, q);
+  cl_barrier();  // x gathered by every CTA before z takes its place
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    const int i = tid + u * kClThreads;
+    if (i < nrow) {
+      r[u] = A.b[r0 + i] - q[u];
+      const double zi = r[u] * jv[u];
+      sz[i] = zi;
+      arr += r[u] * r[u];
+      arz += r[u] * zi;
+    }
   }
   double rr, rho;
-  cluster_totals(0, arr, arz, &rr, &rho);
+  totals(arr, arz, rr, rho);
   const double rnorm0 = sqrt(rr);
   const double thr = fmax(A.st->tol_abs, A.st->tol_rel * rnorm0);
   const int max_iter = A.st->max_iter;
   int iter = 0, term = CFD_TERM_MAX_ITERATIONS;
-  double rn = rnorm0;
+  double rn = rnorm0, beta = 0.0;
   if (!isfinite(rnorm0)) {
     term = CFD_TERM_BREAKDOWN;
   } else if (rnorm0 <= thr) {
     term = CFD_TERM_INITIAL_RESIDUAL;
   } else {
-    for (;;) {
-      cluster.sync();  // p complete in every CTA
-      double apq = 0.0;
-      for (int i = threadIdx.x; i < nrow; i += blockDim.x) {
-        const double qi = row_sum(i, pp);
-        sq[i] = qi;
-        apq += sp[i] * qi;
+    for (int buf = 0;; buf ^= 1) {
+      // p = z + beta p into the other buffer, q = A p
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int i = tid + u * kClThreads;
+        p[u] = fma(beta, p[u], r[u] * jv[u]);
+        if (i < nrow) sp(buf ^ 1)[i] = p[u];
       }
+      __syncthreads();
+      row_sums(buf, beta, q);
+      double apq = 0.0;
+#pragma unroll
+      for (int u = 0; u < R; ++u)
+        if (tid + u * kClThreads < nrow) apq += p[u] * q[u];
       double pq, unused;
-      cluster_totals(1, apq, 0.0, &pq, &unused);
+      totals(apq, 0.0, pq, unused);
       if (!(pq > 0.0)) {
         term = CFD_TERM_NON_POSITIVE_CURVATURE;
         break;
@@ -209,16 +354,23 @@ __global__ void __launch_bounds__(kClThreads) k_cluster_pcg(ClusterArgs A) {
       const double alpha = rho / pq;
       arr = 0.0;
       arz = 0.0;
-      for (int i = threadIdx.x; i < nrow; i += blockDim.x) {
-        sx[i] = sx[i] + alpha * sp[i];
-        const double ri = sr[i] - alpha * sq[i];
-        sr[i] = ri;
-        arr += ri * ri;
-        arz += ri * (ri * sj[i]);
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int i = tid + u * kClThreads;
+        if (i < nrow) {
+          x[u] = x[u] + alpha * p[u];
+          r[u] = r[u] - alpha * q[u];
+          const double zi = r[u] * jv[u];
+          sz[i] = zi;
+          arr += r[u] * r[u];
+          arz += r[u] * zi;
+        }
       }
       double rz;
-      cluster_totals(0, arr, arz, &rr, &rz);
+      totals(arr, arz, rr, rz);
       ++iter;
+      beta = rz / rho;
+      rho = rz;
       rn = sqrt(rr);
       if (!isfinite(rn)) {
         term = CFD_TERM_BREAKDOWN;
@@ -236,13 +388,14 @@ __global__ void __launch_bounds__(kClThreads) k_cluster_pcg(ClusterArgs A) {
         term = CFD_TERM_BREAKDOWN;
         break;
       }
-      const double beta = rz / rho;
-      rho = rz;
-      for (int i = threadIdx.x; i < nrow; i += blockDim.x) sp[i] = sr[i] * sj[i] + beta * sp[i];
     }
   }
-  for (int i = threadIdx.x; i < nrow; i += blockDim.x) A.x[r0 + i] = sx[i];
-  if (rank == 0 && threadIdx.x == 0) {
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    const int i = tid + u * kClThreads;
+    if (i < nrow) A.x[r0 + i] = x[u];
+  }
+  if (rank == 0 && tid == 0) {
     DevState* st = A.st;
     st->rnorm0 = rnorm0;
     st->threshold = thr;
@@ -252,66 +405,73 @@ __global__ void __launch_bounds__(kClThreads) k_cluster_pcg(ClusterArgs A) {
     st->term = term;
     st->done = 1;
   }
-  cluster.sync();  // no CTA leaves while its shared memory may still be read
+  cl_barrier();  // no CTA leaves while its shared memory may still be read
+}
+
+template <int R>
+cfd_status cl_launch(cfd_context* ctx, const ClusterArgs& args, int ncta, size_t bytes, bool* launched) {
+  auto kern = k_cluster_pcg<R>;
+  CFD_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (ncta > 8) CFD_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfgl = {};
+  cfgl.gridDim = dim3(ncta);
+  cfgl.blockDim = dim3(kClThreads);
+  cfgl.dynamicSmemBytes = bytes;
+  cfgl.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ncta;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfgl.attrs = attr;
+  cfgl.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfgl) != cudaSuccess || clusters < 1) {
+    cudaGetLastError();
+    return CFD_OK;
+  }
+  CFD_TRY_CUDA(cudaLaunchKernelEx(&cfgl, kern, args));
+  ctx->stats.launches++;
+  *launched = true;
+  return CFD_OK;
 }
 
 }  // namespace
 
 // The cluster solve applies when the system's rows, split over at most 16
-// CTAs, fit their shared memory; *ok = false otherwise (nothing launched).
-cfd_status cluster_pcg_solve(cfd_context* ctx, const DevMat& m, const double* jinv, const double* b, double* x,
-                             DevState* st, bool* ok) {
+// CTAs, fit their shared memory and registers; *ok = false otherwise (nothing
+// launched).
+cfd_status cluster_pcg_solve(cfd_context* ctx, const HostCsr& h, const DevMat& m, const double* jinv, const double* b,
+                             double* x, DevState* st, bool* ok) {
   *ok = false;
   const int64_t n = m.nrows;
-  if (n <= 0 || n >= (int64_t)kClMaxCtas * 65536 || m.nrows != m.ncols) return CFD_OK;
+  if (n <= 0 || n > (int64_t)kClMaxCtas * kClThreads * kClMaxRows || m.nrows != m.ncols) return CFD_OK;
   int max_smem = 0;
   CFD_TRY_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
   const size_t budget = (size_t)max_smem - 2048;  // static shared arrays
-  // about 1024 rows per CTA (two per thread) where the cluster allows it,
-  // more CTAs where a block does not fit the shared memory
+  // one row per thread where the cluster allows it, more rows per thread at 16 CTAs
   int first = 2;
-  while (first < kClMaxCtas && (n + first - 1) / first > 2 * kClThreads) first *= 2;
-  std::vector<int> rp32;
+  while (first < kClMaxCtas && (n + first - 1) / first > kClThreads) first *= 2;
   for (int ncta = first; ncta <= kClMaxCtas; ncta *= 2) {
     const int rpc = (int)((n + ncta - 1) / ncta);
-    if (rpc >= 65536) continue;
-    if (rp32.empty()) {
-      rp32.resize(n + 1);
-      CFD_TRY_CUDA(cudaMemcpyAsync(rp32.data(), m.rp, (n + 1) * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-      CFD_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
-    }
-    int nnz_cap = 0;
-    for (int c = 0; c < ncta; ++c) {
-      const int64_t a = std::min<int64_t>((int64_t)c * rpc, n), e = std::min<int64_t>((int64_t)(c + 1) * rpc, n);
-      nnz_cap = std::max(nnz_cap, rp32[e] - rp32[a]);
-    }
-    const ClusterLayout L = cluster_layout(rpc, nnz_cap);
+    if (rpc > kClThreads * kClMaxRows) continue;
+    int64_t nnz_cap = 0;
+    for (int64_t r = 0; r < n; r += rpc) nnz_cap = std::max(nnz_cap, h.rp[std::min<int64_t>(r + rpc, n)] - h.rp[r]);
+    const ClusterLayout L = cluster_layout(rpc, (int)std::min<int64_t>(nnz_cap, 1 << 24));
     if (L.bytes > budget) continue;
-    CFD_TRY_CUDA(cudaFuncSetAttribute(k_cluster_pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes));
-    if (ncta > 8)
-      CFD_TRY_CUDA(cudaFuncSetAttribute(k_cluster_pcg, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchConfig_t cfgl = {};
-    cfgl.gridDim = dim3(ncta);
-    cfgl.blockDim = dim3(kClThreads);
-    cfgl.dynamicSmemBytes = L.bytes;
-    cfgl.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ncta;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfgl.attrs = attr;
-    cfgl.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, k_cluster_pcg, &cfgl) != cudaSuccess || clusters < 1) {
-      cudaGetLastError();
-      continue;
-    }
-    ClusterArgs args{m.rp, m.col, m.v64, jinv, b, x, st, (int)n, rpc, nnz_cap};
-    CFD_TRY_CUDA(cudaLaunchKernelEx(&cfgl, k_cluster_pcg, args));
-    ctx->stats.launches++;
-    *ok = true;
-    return CFD_OK;
+    ClusterArgs args{m.rp, m.col, m.v64, jinv, b, x, st, (int)n, rpc, (int)nnz_cap};
+    const int rows = (rpc + kClThreads - 1) / kClThreads;
+    if (rows <= 1)
+      CFD_TRY(cl_launch<1>(ctx, args, ncta, L.bytes, ok));
+    else if (rows <= 2)
+      CFD_TRY(cl_launch<2>(ctx, args, ncta, L.bytes, ok));
+    else if (rows <= 4)
+      CFD_TRY(cl_launch<4>(ctx, args, ncta, L.bytes, ok));
+    else if (rows <= 5)
+      CFD_TRY(cl_launch<5>(ctx, args, ncta, L.bytes, ok));
+    else
+      CFD_TRY(cl_launch<8>(ctx, args, ncta, L.bytes, ok));
+    if (*ok) return CFD_OK;
   }
   return CFD_OK;
 }

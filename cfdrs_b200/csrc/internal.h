@@ -360,8 +360,8 @@ cfd_status ensure_diagonals(cfd_csr* a);
 cfd_status pattern_outer_launch(cfd_csr* a, const double* lambda, const double* x, double scale, double* g);
 // Whole CG / Jacobi-PCG solve in one thread-block cluster (cluster_pcg.cu):
 // *ok = false (nothing launched) when the system does not fit.
-cfd_status cluster_pcg_solve(cfd_context* ctx, const DevMat& m, const double* jinv, const double* b, double* x,
-                             DevState* st, bool* ok);
+cfd_status cluster_pcg_solve(cfd_context* ctx, const HostCsr& h, const DevMat& m, const double* jinv, const double* b,
+                             double* x, DevState* st, bool* ok);
 // Whole GMRES(m) solve (no preconditioner, Jacobi or AMG) in one thread-block
 // cluster (cluster_gmres.cu): *ok = false (nothing launched) when it does not fit.
 cfd_status cluster_gmres_solve(cfd_context* ctx, const cfd_csr* a, cfd_amg* amg, int precond, int m, const double* b,
