@@ -312,7 +312,8 @@ struct cfd_context {
   int* h_err = nullptr;  // pinned mirror
   int num_sms = 148;
   // CG / Jacobi-PCG (cluster_pcg.cu) and FP64 GMRES (cluster_gmres.cu) of small
-  // systems as one thread-block-cluster launch where the system fits;
+  // systems as one thread-block-cluster launch where the system fits, larger CG /
+  // Jacobi-PCG systems on one cooperative grid (grid_pcg.cu) where they fit that;
   // cfd_context_set_cluster_solve
   bool cluster_solve = true;
   cfd::KernelStats stats;
@@ -348,6 +349,9 @@ struct cfd_csr {
   uint64_t values_version = 0;
   cfd_csr* tr = nullptr;
   uint64_t tr_version = 0;
+  // Boundary entries of the fullest row block of the grid CG (grid_pcg.cu), -1
+  // before its first use; a function of the pattern and the GPU's SM count.
+  int64_t grid_far = -1;
 };
 
 namespace cfd {
@@ -362,6 +366,10 @@ cfd_status pattern_outer_launch(cfd_csr* a, const double* lambda, const double* 
 // *ok = false (nothing launched) when the system does not fit.
 cfd_status cluster_pcg_solve(cfd_context* ctx, const HostCsr& h, const DevMat& m, const double* jinv, const double* b,
                              double* x, DevState* st, bool* ok);
+// CG / Jacobi-PCG on one cooperative grid (grid_pcg.cu), for systems beyond a
+// cluster: *ok = false (nothing launched) when the system does not fit.
+cfd_status grid_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, const double* b, double* x, DevState* st,
+                          DevState* host_st, bool* ok);
 // Whole GMRES(m) solve (no preconditioner, Jacobi or AMG) in one thread-block
 // cluster (cluster_gmres.cu): *ok = false (nothing launched) when it does not fit.
 cfd_status cluster_gmres_solve(cfd_context* ctx, const cfd_csr* a, cfd_amg* amg, int precond, int m, const double* b,
