@@ -323,6 +323,373 @@ __global__ void k_batch_pcg(BatchSys S, BatchOut O, const int* __restrict__ orde
   }
 }
 
+// ---- the same solve with the rows in registers --------------------------------
+// What bounded k_batch_pcg: with six vectors in shared memory a system of the
+// largest bucket took 170 KB, one CTA of eight warps per SM, whose iteration is a
+// chain of dependent shared-memory loads and three reductions. Here a thread's R
+// rows (i = t, t + threads, ...) keep x, r, q and the residual scale in registers;
+// shared memory holds the matrix, D^-1 and p (100 KB, two systems per SM), the
+// entries of two rows are read four at a time without branches (slots past a
+// row's end take a zero entry), and r.z and the residual are reduced together.
+// The buckets are parallel branches of the captured graph. Every sum is formed
+// in k_batch_pcg's order, so the results are the same bits. Measured, 768
+// networks of 20 to 2000 nodes to 1e-10: FP64 32.7 -> 15.4 ms, FP32 inside
+// refinement 49.8 -> 25.0 ms. Reading longer rows one at a time instead of two
+// side by side was slower (16.9 ms).
+template <typename T>
+__host__ __device__ constexpr size_t batch_reg_col_off(int zmax) {
+  return round16((size_t)(zmax + 1) * sizeof(T));
+}
+template <typename T>
+__host__ __device__ constexpr size_t batch_reg_rp_off(int zmax) {
+  return batch_reg_col_off<T>(zmax) + round16((size_t)(zmax + 1) * 2);
+}
+template <typename T>
+__host__ __device__ constexpr size_t batch_reg_p_off(int nmax, int zmax) {
+  return batch_reg_rp_off<T>(zmax) + round16((size_t)(nmax + 1) * 2);
+}
+template <typename T>
+__host__ __device__ constexpr size_t batch_reg_smem(int nmax, int zmax) {
+  return batch_reg_p_off<T>(nmax, zmax) + 2 * round16((size_t)nmax * sizeof(T));
+}
+
+// group_sum of two values at once, each in group_sum's order (an exclusive-or
+// butterfly adds the same pairs as the shift-down tree and leaves the sum in
+// every lane; adding the zeros of absent warps is left out).
+__device__ __forceinline__ void group_sum2(double& a, double& b, double (*buf)[32], const Group& G, int groups) {
+  const int lane = G.t & 31, w = G.t >> 5, nw = G.gsz >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  if (nw == 1) return;
+  if (lane == 0) {
+    buf[0][w] = a;
+    buf[1][w] = b;
+  }
+  G.sync(groups);
+  a = buf[0][lane & (nw - 1)];
+  b = buf[1][lane & (nw - 1)];
+  for (int o = nw >> 1; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+}
+
+constexpr int kRegThreads = 512;  // threads of a CTA at most (128 registers each)
+
+template <typename T, bool REFINE, int R>
+__global__ void __launch_bounds__(kRegThreads) k_batch_pcg_reg(BatchSys S, BatchOut O, const int* __restrict__ order,
+                                                               int count, unsigned* queue,
+                                                               const BatchParams* __restrict__ prm, int nmax,
+                                                               int zmax, int groups) {
+  extern __shared__ __align__(16) unsigned char smem_all[];
+  const Group G(groups);
+  unsigned char* sm = smem_all + (size_t)G.g * round16(batch_reg_smem<T>(nmax, zmax));
+  T* sv = reinterpret_cast<T*>(sm);
+  unsigned short* sc = reinterpret_cast<unsigned short*>(sm + batch_reg_col_off<T>(zmax));
+  unsigned short* srp = reinterpret_cast<unsigned short*>(sm + batch_reg_rp_off<T>(zmax));
+  T* vp = reinterpret_cast<T*>(sm + batch_reg_p_off<T>(nmax, zmax));
+  T* vj = reinterpret_cast<T*>(sm + batch_reg_p_off<T>(nmax, zmax) + round16((size_t)nmax * sizeof(T)));
+  __shared__ double reds[kMaxGroups][2][2][32];
+  __shared__ int s_ks[kMaxGroups];
+  double(*red)[2][32] = reds[G.g];
+  int& s_k = s_ks[G.g];
+  const int tid = G.t, nt = G.gsz;
+  const BatchParams P = *prm;
+  auto gsync = [&]() { G.sync(groups); };
+  constexpr int U = 4;                 // entries of a row read together
+  constexpr int V = R >= 2 ? 2 : 1;    // rows side by side
+  T x[R], r[R], q[R], es[R];           // es: equilibration scale 1 / max_j |a_ij|
+
+  for (;;) {
+    if (tid == 0) s_k = (int)atomicAdd(queue, 1u);
+    gsync();
+    const int k = s_k;
+    gsync();
+    if (k >= count) break;
+    const int sys = order[k];
+    const int r0 = S.sys_row[sys], n = S.sys_row[sys + 1] - r0;
+    const int k0 = S.rp[r0], nnz = S.rp[r0 + n] - k0;
+    // ---- stage the system ----
+    for (int i = tid; i <= n; i += nt) srp[i] = (unsigned short)(S.rp[r0 + i] - k0);
+    for (int e = tid; e < nnz; e += nt) {
+      sv[e] = REFINE ? (T)S.v32[k0 + e] : (T)S.v64[k0 + e];
+      sc[e] = (unsigned short)S.col[k0 + e];
+    }
+    if (tid == 0) {  // the zero entry: row 0's direction times 0
+      sv[zmax] = T(0);
+      sc[zmax] = 0;
+      vp[0] = T(0);
+    }
+    gsync();
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const int i = tid + u * nt;
+      es[u] = x[u] = r[u] = q[u] = T(0);
+      if (i < n) {
+        double d = 0.0, mx = 0.0;
+        for (int e = srp[i]; e < srp[i + 1]; ++e) {
+          const double a = REFINE ? (double)S.v64[k0 + e] : (double)sv[e];
+          if (sc[e] == i) d = a;
+          mx = fmax(mx, fabs(a));
+        }
+        vj[i] = (T)(fabs(d) <= DBL_EPSILON ? 1.0 : 1.0 / d);
+        es[u] = (T)((mx > DBL_EPSILON && isfinite(mx)) ? 1.0 / mx : 1.0);
+      }
+    }
+    gsync();
+    int term = CFD_TERM_MAX_ITERATIONS, it_total = 0;
+    double e_rel = 0.0;
+    int slot = 0;
+    auto sum2 = [&](double& a, double& b) {
+      group_sum2(a, b, red[slot], G, groups);
+      slot ^= 1;
+    };
+    // y = A p for this thread's rows (p in vp)
+    auto spmv = [&](T (&y)[R]) {
+#pragma unroll
+      for (int u0 = 0; u0 < R; u0 += V) {
+        int ka[V], ke[V];
+        T s[V];
+        bool more = false;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const int i = min(tid + (u0 + v) * nt, n);  // row n: empty
+          ka[v] = srp[i];
+          ke[v] = srp[min(i + 1, n)];
+          s[v] = T(0);
+          more |= ka[v] < ke[v];
+        }
+        while (more) {
+          T a[V][U], p[V][U];
+          more = false;
+#pragma unroll
+          for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int w = 0; w < U; ++w) {
+              const int e = ka[v] + w < ke[v] ? ka[v] + w : zmax;
+              a[v][w] = sv[e];
+              p[v][w] = vp[sc[e]];
+            }
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+#pragma unroll
+            for (int w = 0; w < U; ++w) s[v] += a[v][w] * p[v][w];
+            ka[v] += U;
+            more |= ka[v] < ke[v];
+          }
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) y[u0 + v] = s[v];
+      }
+    };
+    // Inner PCG on (A, rhs in r) from x; returns iterations; sets term.
+    auto pcg = [&](double thr_rel, int max_it, double& e0_out, double& e_out, int& term_out, bool abs_thr,
+                   double thr_abs) {
+      double rho = 0.0, e2 = 0.0;
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int i = tid + u * nt;
+        if (i < n) {
+          const T ri = r[u];
+          const T zi = ri * vj[i];
+          vp[i] = zi;
+          rho += (double)ri * (double)zi;
+          const double si = (double)es[u] * (double)ri;
+          e2 += si * si;
+        }
+      }
+      sum2(rho, e2);
+      const double e0 = sqrt(e2);
+      e0_out = e0;
+      e_out = e0;
+      const double thr = abs_thr ? fmax(thr_abs, thr_rel * e0) : thr_rel * e0;
+      if (!isfinite(e0)) {
+        term_out = CFD_TERM_BREAKDOWN;
+        return 0;
+      }
+      if (e0 <= thr) {
+        term_out = CFD_TERM_INITIAL_RESIDUAL;
+        return 0;
+      }
+      gsync();
+      for (int it = 1; it <= max_it; ++it) {
+        double pq = 0.0, none = 0.0;
+        spmv(q);
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          const int i = tid + u * nt;
+          if (i < n) pq += (double)vp[i] * (double)q[u];
+        }
+        sum2(pq, none);
+        if (!(pq > 0.0)) {
+          term_out = CFD_TERM_NON_POSITIVE_CURVATURE;
+          return it - 1;
+        }
+        const T alpha = (T)(rho / pq);
+        double rz = 0.0;
+        e2 = 0.0;
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          const int i = tid + u * nt;
+          if (i < n) {
+            x[u] = x[u] + alpha * vp[i];
+            const T ri = r[u] - alpha * q[u];
+            r[u] = ri;
+            rz += (double)ri * (double)(ri * vj[i]);
+            const double si = (double)es[u] * (double)ri;
+            e2 += si * si;
+          }
+        }
+        sum2(rz, e2);
+        const double e = sqrt(e2);
+        e_out = e;
+        if (!isfinite(e)) {
+          term_out = CFD_TERM_BREAKDOWN;
+          return it;
+        }
+        if (e <= thr) {
+          term_out = CFD_TERM_CONVERGED;
+          return it;
+        }
+        if (rz == 0.0 || !isfinite(rz)) {
+          term_out = CFD_TERM_BREAKDOWN;
+          return it;
+        }
+        const T beta = (T)(rz / rho);
+        rho = rz;
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          const int i = tid + u * nt;
+          if (i < n) vp[i] = r[u] * vj[i] + beta * vp[i];
+        }
+        gsync();
+      }
+      term_out = CFD_TERM_MAX_ITERATIONS;
+      return max_it;
+    };
+
+    if (!REFINE) {
+      // r = b - A x0, x0 gathered from vp
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int i = tid + u * nt;
+        if (i < n) {
+          x[u] = (T)O.x[r0 + i];
+          vp[i] = x[u];
+        }
+      }
+      gsync();
+      spmv(q);
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int i = tid + u * nt;
+        if (i < n) r[u] = (T)O.b[r0 + i] - q[u];
+      }
+      gsync();
+      double e0, e;
+      it_total = pcg(P.tol_rel, P.max_iter, e0, e, term, true, P.tol_abs);
+      e_rel = e0 > 0.0 ? e / e0 : 0.0;
+      gsync();
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int i = tid + u * nt;
+        if (i < n) O.x[r0 + i] = (double)x[u];
+      }
+    } else {
+      // Outer FP64 residual and update from global memory, inner FP32 PCG.
+      double e_first = -1.0, thr = 0.0;
+      term = CFD_TERM_MAX_ITERATIONS;
+      for (int outer = 0; outer <= P.max_outer; ++outer) {
+        double r2 = 0.0, e2 = 0.0;
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          const int i = tid + u * nt;
+          if (i < n) {
+            double s = 0.0;
+            for (int e = srp[i]; e < srp[i + 1]; ++e) s += S.v64[k0 + e] * O.x[r0 + sc[e]];
+            const double ri = O.b[r0 + i] - s;
+            r2 += ri * ri;
+            const double si = (double)es[u] * ri;
+            e2 += si * si;
+          }
+        }
+        sum2(r2, e2);
+        const double e = sqrt(e2), rn = sqrt(r2);
+        if (e_first < 0.0) {
+          e_first = e;
+          thr = fmax(P.tol_abs, P.tol_rel * e);
+        }
+        e_rel = e_first > 0.0 ? e / e_first : 0.0;
+        if (!isfinite(e)) {
+          term = CFD_TERM_BREAKDOWN;
+          break;
+        }
+        if (e <= thr) {
+          term = (outer == 0) ? CFD_TERM_INITIAL_RESIDUAL : CFD_TERM_CONVERGED;
+          break;
+        }
+        if (outer == P.max_outer || it_total >= P.max_iter) break;
+        const double scale = 1.0 / rn;
+        gsync();
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          const int i = tid + u * nt;
+          if (i < n) {
+            double s = 0.0;
+            for (int e2i = srp[i]; e2i < srp[i + 1]; ++e2i) s += S.v64[k0 + e2i] * O.x[r0 + sc[e2i]];
+            r[u] = (T)((O.b[r0 + i] - s) * scale);
+            x[u] = T(0);
+          }
+        }
+        gsync();
+        double ie0, ie;
+        int iterm = CFD_TERM_MAX_ITERATIONS;
+        const int its = pcg(P.inner_tol, P.max_iter - it_total, ie0, ie, iterm, false, 0.0);
+        it_total += its;
+        gsync();
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          const int i = tid + u * nt;
+          if (i < n) O.x[r0 + i] += (double)x[u] / scale;
+        }
+        gsync();
+        if (iterm == CFD_TERM_BREAKDOWN || iterm == CFD_TERM_NON_POSITIVE_CURVATURE) {
+          term = iterm;
+          break;
+        }
+      }
+    }
+    if (tid == 0) {
+      O.term[sys] = term;
+      O.iters[sys] = it_total;
+      O.resid[sys] = e_rel;
+    }
+    gsync();
+  }
+}
+
+using BatchKernel = void (*)(BatchSys, BatchOut, const int*, int, unsigned*, const BatchParams*, int, int, int);
+
+// The kernel of a bucket: rows in registers up to eight rows a thread and 512
+// threads a CTA, else the vectors in shared memory (which other thread counts,
+// chosen by autotune or the caller, may ask for).
+template <typename T, bool REFINE>
+BatchKernel batch_kernel(int nmax, int zmax, int threads, int groups, size_t* smem) {
+  const int rows = (nmax + threads - 1) / threads;
+  if (threads * groups <= kRegThreads && rows <= 8) {
+    *smem = (size_t)groups * round16(batch_reg_smem<T>(nmax, zmax));
+    if (rows <= 1) return k_batch_pcg_reg<T, REFINE, 1>;
+    if (rows <= 2) return k_batch_pcg_reg<T, REFINE, 2>;
+    if (rows <= 4) return k_batch_pcg_reg<T, REFINE, 4>;
+    return k_batch_pcg_reg<T, REFINE, 8>;
+  }
+  *smem = (size_t)groups * round16(batch_smem<T>(nmax, zmax));
+  return k_batch_pcg<T, REFINE>;
+}
+
 }  // namespace
 }  // namespace cfd
 
@@ -348,10 +715,22 @@ cfd_status prepare_bucket(cfd_batch* bt, int bkt, int threads, int groups, int* 
   const int count = bt->bucket_begin[bkt + 1] - bt->bucket_begin[bkt];
   *grid = 0;
   if (count == 0) return CFD_OK;
-  const size_t smem = (size_t)groups * round16(batch_smem<T>(bt->bucket_nmax[bkt], bt->bucket_zmax[bkt]));
+  size_t smem = 0;
+  const BatchKernel kern =
+      batch_kernel<T, REFINE>(bt->bucket_nmax[bkt], bt->bucket_zmax[bkt], threads, groups, &smem);
   threads *= groups;
-  auto kern = k_batch_pcg<T, REFINE>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  // The limit of the device, not of this bucket: buckets (and batches) share
+  // kernels, and a graph may be replayed after another bucket was prepared.
+  cudaFuncAttributes fa;
+  int optin = 0;
+  CFD_TRY_CUDA(cudaFuncGetAttributes(&fa, kern));
+  CFD_TRY_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, bt->ctx->device));
+  const size_t limit = (size_t)optin - fa.sharedSizeBytes;
+  // a configuration is accepted by the larger form's need, whichever form runs
+  const size_t need =
+      std::max(smem, (size_t)groups * round16(batch_smem<T>(bt->bucket_nmax[bkt], bt->bucket_zmax[bkt])));
+  if (need > limit || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) !=
+                          cudaSuccess) {
     cudaGetLastError();
     set_error("batch bucket %d: %zu bytes of shared memory are not available", bkt, smem);
     return CFD_ERR_CONFIG;
@@ -374,9 +753,11 @@ cfd_status launch_bucket(cfd_batch* bt, int bkt, int threads, int groups, int gr
   if (count == 0 || grid == 0) return CFD_OK;
   BatchSys S{bt->sys_row, bt->rp, bt->col, bt->v64, bt->v32};
   BatchOut O{bt->x, bt->b, bt->term, bt->iters, bt->resid};
-  k_batch_pcg<T, REFINE><<<grid, threads * groups, smem, s>>>(S, O, bt->order + bt->bucket_begin[bkt], count,
-                                                               bt->queues + bkt, bt->params, bt->bucket_nmax[bkt],
-                                                               bt->bucket_zmax[bkt], groups);
+  size_t same = 0;
+  const BatchKernel kern =
+      batch_kernel<T, REFINE>(bt->bucket_nmax[bkt], bt->bucket_zmax[bkt], threads, groups, &same);
+  kern<<<grid, threads * groups, smem, s>>>(S, O, bt->order + bt->bucket_begin[bkt], count, bt->queues + bkt,
+                                            bt->params, bt->bucket_nmax[bkt], bt->bucket_zmax[bkt], groups);
   CFD_TRY_CUDA(cudaGetLastError());
   return CFD_OK;
 }
@@ -389,15 +770,24 @@ cfd_status run_bucket(cfd_batch* bt, int bkt, int threads, int groups, cudaStrea
   return launch_bucket<REFINE>(bt, bkt, threads, groups, grid, smem, s);
 }
 
-// The device part of one batched solve: reset the queues, one persistent
-// launch per bucket (largest systems first).
-cfd_status enqueue_solve(cfd_batch* bt, int prec, const int* grid, const size_t* smem, cudaStream_t s) {
+// The device part of one batched solve: reset the queues, then one persistent
+// launch per bucket, each on a stream of its own between a fork and a join
+// (largest systems first).
+cfd_status enqueue_solve(cfd_batch* bt, int prec, const int* grid, const size_t* smem, cudaStream_t s,
+                         const cudaStream_t* branch, const cudaEvent_t* ev) {
   CFD_TRY_CUDA(cudaMemsetAsync(bt->queues, 0, kBuckets * sizeof(unsigned), s));
+  CFD_TRY_CUDA(cudaEventRecord(ev[0], s));
   for (int k = kBuckets - 1; k >= 0; --k) {
+    if (k > 0) CFD_TRY_CUDA(cudaStreamWaitEvent(branch[k], ev[0], 0));
+    cudaStream_t q = k > 0 ? branch[k] : s;
     if (prec)
-      CFD_TRY(launch_bucket<true>(bt, k, bt->threads[prec][k], bt->groups[prec][k], grid[k], smem[k], s));
+      CFD_TRY(launch_bucket<true>(bt, k, bt->threads[prec][k], bt->groups[prec][k], grid[k], smem[k], q));
     else
-      CFD_TRY(launch_bucket<false>(bt, k, bt->threads[prec][k], bt->groups[prec][k], grid[k], smem[k], s));
+      CFD_TRY(launch_bucket<false>(bt, k, bt->threads[prec][k], bt->groups[prec][k], grid[k], smem[k], q));
+  }
+  for (int k = kBuckets - 1; k > 0; --k) {
+    CFD_TRY_CUDA(cudaEventRecord(ev[k], branch[k]));
+    CFD_TRY_CUDA(cudaStreamWaitEvent(s, ev[k], 0));
   }
   return CFD_OK;
 }
@@ -416,25 +806,25 @@ cfd_status capture_graph(cfd_batch* bt, int prec) {
     else
       CFD_TRY(prepare_bucket<false>(bt, k, bt->threads[prec][k], bt->groups[prec][k], &grid[k], &smem[k]));
   }
-  // The buckets share one kernel per precision: its shared-memory limit must
-  // cover the largest of them (with several systems per CTA a small-row
-  // bucket can need more than a larger one).
-  const size_t smem_max = *std::max_element(smem, smem + kBuckets);
-  if (smem_max > 0) {
-    const cudaError_t ea =
-        prec ? cudaFuncSetAttribute(k_batch_pcg<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem_max)
-             : cudaFuncSetAttribute(k_batch_pcg<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem_max);
-    if (ea != cudaSuccess) {
-      cudaGetLastError();
-      set_error("batch: %zu bytes of shared memory are not available", smem_max);
-      return CFD_ERR_CONFIG;
+  // The buckets are parallel branches: a bucket's CTAs start where the larger
+  // ones' queue has run dry.
+  struct Branches {
+    cudaStream_t s[kBuckets] = {};
+    cudaEvent_t e[kBuckets] = {};
+    ~Branches() {
+      for (int k = 0; k < kBuckets; ++k) {
+        if (e[k]) cudaEventDestroy(e[k]);
+        if (s[k]) cudaStreamDestroy(s[k]);
+      }
     }
+  } br;
+  for (int k = 0; k < kBuckets; ++k) {
+    CFD_TRY_CUDA(cudaStreamCreateWithFlags(&br.s[k], cudaStreamNonBlocking));
+    CFD_TRY_CUDA(cudaEventCreateWithFlags(&br.e[k], cudaEventDisableTiming));
   }
   cudaGraph_t g = nullptr;
   CFD_TRY_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  cfd_status st = enqueue_solve(bt, prec, grid, smem, s);
+  cfd_status st = enqueue_solve(bt, prec, grid, smem, s, br.s, br.e);
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (st != CFD_OK) {
     if (g) cudaGraphDestroy(g);

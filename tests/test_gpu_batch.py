@@ -140,3 +140,39 @@ def test_batch_set_config_rejects_bad_widths(batch):
         nb.set_config([512, 64, 64, 64], [4, 1, 1, 1])
     with pytest.raises(_lib.CfdError):
         nb.set_config([64, 64, 64, 64], [3, 1, 1, 1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_refine"])
+def test_rows_in_registers_match_shared_memory_vectors(cuda, precision):
+    """The register form (up to 8 rows a thread and 512 threads a CTA) and the
+    shared-memory form (beyond) of the Jacobi-PCG kernel form every sum in the
+    same order: with the same threads per system their results are the same
+    bits. Sizes around 1, 2, 4 and 8 rows of 32 threads a thread; four systems
+    of 256 threads force the shared-memory form."""
+    import cfdrs_b200 as cf
+    from cfdrs_b200 import problems as P
+    from cfdrs_b200.batch import NetworkBatch
+    rng = np.random.default_rng(11)
+    prec = cf.Precision.FP64 if precision == "fp64" else cf.Precision.FP32_REFINE
+    cfg = cf.IterativeSolverConfig(0.0, 1e-10, 20000)
+    for sizes in ([2, 3, 31, 32, 33, 63, 64], [65, 127, 128, 129, 200, 255, 256]):
+        systems = [P.random_network(n, rng) for n in sizes]
+        b = np.concatenate([q for _, q in systems])
+        nb = NetworkBatch([A for A, _ in systems])
+        got = []
+        for groups in (1, 4):  # 256 threads x 4 systems = 1024 threads: the shared-memory form
+            nb.set_config([256, 256, 256, 256], [groups] * 4, prec)
+            got.append(nb.solve(b, config=cfg, precision=prec))
+        (x1, r1), (x2, r2) = got
+        np.testing.assert_array_equal(x1, x2)
+        np.testing.assert_array_equal(r1.iterations, r2.iterations)
+        np.testing.assert_array_equal(r1.termination, r2.termination)
+        # 32 threads: 2 to 8 rows a thread against four systems a CTA of the same width
+        got = []
+        for groups in (1, 4):
+            nb.set_config([32, 32, 32, 32], [groups] * 4, prec)
+            got.append(nb.solve(b, config=cfg, precision=prec))
+        (x1, r1), (x2, r2) = got
+        np.testing.assert_array_equal(x1, x2)
+        for (A, _), xs, bs in zip(systems, nb.split(x1), nb.split(b)):
+            assert eq_residual(A, xs, bs) <= 1.5e-10
