@@ -1223,7 +1223,8 @@ cfd_status cfd_batch_destroy(cfd_batch* bt) {
                   (void*)bt->b, (void*)bt->term, (void*)bt->iters, (void*)bt->resid, (void*)bt->order,
                   (void*)bt->queues, (void*)bt->params, (void*)bt->ls_method, (void*)bt->ls_path,
                   (void*)bt->ls_list, (void*)bt->ls_params, (void*)bt->ls_queue, (void*)bt->ls_scratch,
-                  (void*)bt->ls_pivot})
+                  (void*)bt->ls_pivot, (void*)bt->ls_plan_heads, (void*)bt->ls_plan_rounds,
+                  (void*)bt->ls_plan_words, (void*)bt->ls_plan_init})
     if (p) cudaFree(p);
   if (bt->h_params) cudaFreeHost(bt->h_params);
   network_plan_free(bt->net);

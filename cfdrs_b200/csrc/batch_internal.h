@@ -22,6 +22,8 @@ struct BatchParams {
 };
 
 struct NetworkPlanDev;  // network.cu
+struct LsPlanHead;      // ls_plan.h
+struct LsRound;
 
 // Checks a batch layout (offsets, row_ptr, local columns) without touching
 // any device state; see cfd_batch_create.
@@ -82,4 +84,11 @@ struct cfd_batch {
   size_t ls_scratch_elems = 0;
   int* ls_pivot = nullptr;   // per system: the dense fast path's pivot guard fired
   int64_t ls_pivoted = 0;    // systems handed to the pivoting dense solve, all calls
+  // Elimination plans (ls_plan.h), made from the pattern at the first direct
+  // solve; core sizes per system, -1: no plan.
+  cfd::LsPlanHead* ls_plan_heads = nullptr;
+  cfd::LsRound* ls_plan_rounds = nullptr;
+  uint16_t* ls_plan_words = nullptr;
+  uint16_t* ls_plan_init = nullptr;
+  std::vector<int> ls_plan_core;
 };

@@ -20,7 +20,9 @@
 // right-looking with partial pivoting (k_ls_dense): 32-column panels factored
 // in place, the trailing matrix updated by 64 x 64 tiles staged in shared
 // memory. The systems whose Krylov solve is not kept are collected on the
-// host after the Krylov launches and solved by a second dense launch.
+// host after the Krylov launches and solved directly: by sparse elimination with
+// a dense core where the pattern has such an order (k_ls_sparse, ls_plan.h), the
+// others, and those that need row exchanges, by a second dense launch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -33,6 +35,7 @@
 #include "batch_internal.h"
 #include "internal.h"
 #include "kernels.cuh"
+#include "ls_plan.h"
 
 namespace cfd {
 namespace {
@@ -926,6 +929,142 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_dense_fast(LsArgs A, const in
   }
 }
 
+// ---- direct solves by sparse elimination ---------------------------------------
+// Solves of the original system along the pattern's elimination plan
+// (ls_plan.h): a network of 2000 nodes and 200 loops is 8 rounds of
+// independent nodes and a core of about 130 unknowns, where the dense LU spends
+// 5 GFLOP on it. One CTA per system: the slots in shared memory, the rounds'
+// lists read once from global memory (their targets differ within a round, and
+// every target adds its products in list order, so results do not depend on
+// scheduling); then the slots move to the CTA's global scratch while
+// lu_solve_fast has the shared memory for the core, and come back for the
+// substitution, rounds in reverse. Pivots are diagonal, as on the dense fast
+// path, with the same guard: a multiplier above 1 by more than rounding, or a
+// zero or non-finite pivot, marks the system for the dense path
+// (pivot[sys] = 1). The direct branch's systems go the same way: their
+// equilibrated matrix is the original with its rows scaled, whose elimination with
+// the same pivots is the original's with every step scaled, so the guard looks at
+// the original's multipliers (the scaled ones pass 1 on nearly every network and
+// sent it to the pivoting kernel); the solution is kept as the equilibrated one
+// when its residual target holds, else as the original's (linear_system.rs:124-130).
+// Measured on 512 networks: 448 fallback systems of 257 to 2000 nodes 76.6 -> 0.6
+// ms, 64 direct ones 3.6 -> 0.1 ms.
+struct SparsePlans {
+  const LsPlanHead* __restrict__ head;
+  const LsRound* __restrict__ rounds;
+  const uint16_t* __restrict__ words;
+  const uint16_t* __restrict__ init;  // slot of every stored entry of the batch
+};
+
+__global__ void __launch_bounds__(kLsThreads) k_ls_sparse(LsArgs A, SparsePlans S, const int* __restrict__ list,
+                                                          int count, int direct, unsigned* queue, double* scratch,
+                                                          size_t slot_elems, const LsParams* __restrict__ prm,
+                                                          int* pivot) {
+  extern __shared__ __align__(16) unsigned char fsm[];
+  double* v = reinterpret_cast<double*>(fsm);
+  __shared__ double red[2][2][32];
+  __shared__ double s_tmp[kFb];
+  __shared__ int s_k, s_bad;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  double* mine = scratch + (size_t)blockIdx.x * slot_elems;
+  int rslot = 0;
+  for (;;) {
+    if (tid == 0) {
+      s_k = (int)atomicAdd(queue, 1u);
+      s_bad = 0;
+    }
+    __syncthreads();
+    const int q = s_k;
+    __syncthreads();
+    if (q >= count) break;
+    const int sys = list[q];
+    const LsPlanHead H = S.head[sys];
+    const uint16_t* w = S.words + H.words;
+    const int r0 = A.sys_row[sys], n = A.sys_row[sys + 1] - r0;
+    for (int i = tid; i < H.slots; i += nt) v[i] = 0.0;
+    __syncthreads();
+    for (int i = tid; i < n; i += nt) {
+      for (int e = A.rp[r0 + i]; e < A.rp[r0 + i + 1]; ++e) v[S.init[e]] += A.v64[e];  // a row's slots are its own
+      v[H.b0 + i] = A.b[r0 + i];
+    }
+    __syncthreads();
+    for (int r = 0; r < H.rounds; ++r) {
+      const LsRound R = S.rounds[H.round0 + r];
+      for (int k = tid; k < R.nl; k += nt) {
+        const int l = w[R.at_l + 2 * k];
+        const double d = v[w[R.at_l + 2 * k + 1]], m = v[l] / d;
+        if (!(fabs(m) <= 1.0 + kPivotSlack) || !isfinite(d)) s_bad = 1;  // a zero or NaN pivot fails the first
+        v[l] = m;
+      }
+      __syncthreads();
+      for (int k = tid; k < R.nt; k += nt) {
+        const int t = w[R.at_t + 3 * k], c = w[R.at_t + 3 * k + 2];
+        const uint16_t* p = w + R.pairs + 2 * (int)w[R.at_t + 3 * k + 1];
+        double s = v[t];
+        for (int u = 0; u < c; ++u) s -= v[p[2 * u]] * v[p[2 * u + 1]];
+        v[t] = s;
+      }
+      __syncthreads();
+    }
+    // the core's matrix and right-hand side, and the slots' stay in global memory
+    double* M = mine + kLsPlanMaxSlots;
+    const int c = H.core;
+    const size_t ld = (size_t)c + 1;
+    for (int i = tid; i < H.slots; i += nt) mine[i] = v[i];
+    for (size_t e = tid; e < (size_t)c * ld; e += nt) M[e] = 0.0;
+    __syncthreads();
+    for (int k = tid; k < H.entries; k += nt) {
+      const uint16_t* e = w + H.at_entries + 3 * k;
+      M[(size_t)e[1] * ld + e[2]] = v[e[0]];
+    }
+    for (int k = tid; k < c; k += nt) M[(size_t)k * ld + c] = v[H.b0 + w[H.at_core + k]];
+    bool bad = s_bad != 0;  // set before the rounds' last barrier
+    __syncthreads();
+    if (!bad && c > 0) bad = !lu_solve_fast(M, M + (size_t)c * ld, c, fsm, &s_bad, s_tmp);
+    __syncthreads();
+    for (int i = tid; i < H.slots; i += nt) v[i] = mine[i];
+    __syncthreads();
+    if (!bad && c > 0)
+      for (int k = tid; k < c; k += nt) v[H.b0 + w[H.at_core + k]] = M[(size_t)k * ld + c];
+    __syncthreads();
+    for (int r = H.rounds - 1; r >= 0 && !bad; --r) {
+      const LsRound R = S.rounds[H.round0 + r];
+      for (int k = tid; k < R.nx; k += nt) {
+        const uint16_t* x = w + R.at_x + 4 * k;
+        const uint16_t* p = w + R.xpairs + 2 * (int)x[2];
+        double s = v[x[0]];
+        for (int u = 0; u < (int)x[3]; ++u) s -= v[p[2 * u]] * v[p[2 * u + 1]];
+        v[x[0]] = s / v[x[1]];
+      }
+      __syncthreads();
+    }
+    // an isolated node has no multiplier: its pivot shows here
+    int nonfinite = 0;
+    if (!bad)
+      for (int i = tid; i < n; i += nt)
+        if (!isfinite(v[H.b0 + i])) nonfinite = 1;
+    bad = __syncthreads_or(nonfinite) || bad;
+    double ratio = NAN;
+    if (!bad) {
+      for (int i = tid; i < n; i += nt) A.x[r0 + i] = v[H.b0 + i];
+      __syncthreads();
+      ratio = ls_target_ratio(A, r0, n, red, rslot);
+    }
+    if (tid == 0) {
+      pivot[sys] = bad ? 1 : 0;
+      if (!bad) {
+        A.resid[sys] = ratio;
+        if (direct) {
+          A.path[sys] = ratio <= prm->tol ? CFD_LS_PATH_DIRECT : CFD_LS_PATH_DIRECT_UNSCALED;
+          A.term[sys] = -1;
+          A.iters[sys] = 0;
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
 // Detection alone for the direct systems (the method is reported for every system).
 __global__ void k_ls_detect(LsArgs A, const int* __restrict__ list, int count, int fixed) {
   const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -1042,6 +1181,117 @@ cfd_status ls_dense_launch(cfd_batch* bt, const LsArgs& A, const std::vector<int
   return CFD_OK;
 }
 
+// The elimination plans, made from the batch's pattern at its first direct solve.
+cfd_status ls_ensure_plans(cfd_batch* bt, cudaStream_t s) {
+  if (bt->ls_plan_heads) return CFD_OK;
+  std::vector<int> rp(bt->rows + 1), col(bt->nnz);
+  CFD_TRY_CUDA(cudaMemcpyAsync(rp.data(), bt->rp, rp.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+  CFD_TRY_CUDA(cudaMemcpyAsync(col.data(), bt->col, col.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+  CFD_TRY_CUDA(cudaStreamSynchronize(s));
+  const int todo = bt->nsys;
+  std::vector<LsPlanOne> plans(todo);
+  int failed = 0;
+#pragma omp parallel for schedule(dynamic, 4)
+  for (int q = 0; q < todo; ++q) {
+    try {  // no exception leaves the parallel region
+      const int sy = bt->h_order[q], r0 = bt->h_sys_row[sy];
+      ls_plan_build(bt->h_sys_row[sy + 1] - r0, rp.data() + r0, col.data(), plans[q]);
+    } catch (...) {
+#pragma omp atomic write
+      failed = 1;
+    }
+  }
+  if (failed) {
+    set_error("cfd_batch_linear_system_solve: host memory for the elimination plans");
+    return CFD_ERR_ALLOC;
+  }
+  std::vector<LsPlanHead> heads(bt->nsys);
+  std::vector<LsRound> rounds;
+  std::vector<uint16_t> init(bt->nnz, 0), words;
+  bt->ls_plan_core.assign(bt->nsys, -1);
+  for (int q = 0; q < todo; ++q) {
+    const int sy = bt->h_order[q];
+    LsPlanOne& P = plans[q];
+    if (!P.head.ok) continue;
+    P.head.words = (int64_t)words.size();
+    P.head.round0 = (int32_t)rounds.size();
+    words.insert(words.end(), P.words.begin(), P.words.end());
+    rounds.insert(rounds.end(), P.rounds.begin(), P.rounds.end());
+    std::copy(P.init.begin(), P.init.end(), init.begin() + rp[bt->h_sys_row[sy]]);
+    heads[sy] = P.head;
+    bt->ls_plan_core[sy] = P.head.core;
+    P = LsPlanOne{};
+  }
+  cfd_status st = ls_alloc(&bt->ls_plan_words, (int64_t)words.size());
+  if (st == CFD_OK) st = ls_alloc(&bt->ls_plan_init, (int64_t)init.size());
+  if (st == CFD_OK) st = ls_alloc(&bt->ls_plan_rounds, (int64_t)rounds.size());
+  LsPlanHead* dev = nullptr;
+  if (st == CFD_OK) st = ls_alloc(&dev, (int64_t)heads.size());
+  auto up = [&](void* d, const void* h, size_t bytes) {
+    if (st == CFD_OK && bytes > 0 && cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess) {
+      set_error("cfd_batch_linear_system_solve: upload of the elimination plans failed");
+      st = CFD_ERR_CUDA;
+    }
+  };
+  up(bt->ls_plan_words, words.data(), words.size() * sizeof(uint16_t));
+  up(bt->ls_plan_init, init.data(), init.size() * sizeof(uint16_t));
+  up(bt->ls_plan_rounds, rounds.data(), rounds.size() * sizeof(LsRound));
+  up(dev, heads.data(), heads.size() * sizeof(LsPlanHead));
+  if (st == CFD_OK && cudaStreamSynchronize(s) != cudaSuccess) st = CFD_ERR_CUDA;
+  if (st != CFD_OK) {
+    for (void* p : {(void*)bt->ls_plan_words, (void*)bt->ls_plan_init, (void*)bt->ls_plan_rounds, (void*)dev})
+      if (p) cudaFree(p);
+    bt->ls_plan_words = bt->ls_plan_init = nullptr;
+    bt->ls_plan_rounds = nullptr;
+    return st;
+  }
+  bt->ls_plan_heads = dev;
+  return CFD_OK;
+}
+
+// Direct solves of the systems in `list` (modes as k_ls_dense): sparse elimination
+// where the pattern has a plan, then the dense path for the rest and for the
+// systems whose pivot guard fired.
+cfd_status ls_direct_launch(cfd_batch* bt, const LsArgs& A, const std::vector<int>& list, bool direct,
+                            cudaStream_t s) {
+  if (list.empty()) return CFD_OK;
+  CFD_TRY(ls_ensure_plans(bt, s));
+  std::vector<int> sparse, dense;
+  int cmax = 0;
+  for (int sy : list) {
+    if (bt->ls_plan_core[sy] < 0) {
+      dense.push_back(sy);
+      continue;
+    }
+    sparse.push_back(sy);
+    cmax = std::max(cmax, bt->ls_plan_core[sy]);
+  }
+  if (!sparse.empty()) {
+    static_assert(kLsPlanMaxSlots * sizeof(double) <= kFastSmem, "the slots fit the core's shared memory");
+    CFD_TRY_CUDA(cudaFuncSetAttribute(k_ls_sparse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFastSmem));
+    const int grid = std::min<int>((int)sparse.size(), bt->ctx->num_sms);
+    const size_t slot = kLsPlanMaxSlots + fast_slot_elems(std::max(cmax, 1));
+    CFD_TRY(ls_ensure_scratch(bt, slot, grid));
+    CFD_TRY_CUDA(
+        cudaMemcpyAsync(bt->ls_list, sparse.data(), sparse.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    CFD_TRY_CUDA(cudaMemsetAsync(bt->ls_queue, 0, sizeof(unsigned), s));
+    const SparsePlans S{bt->ls_plan_heads, bt->ls_plan_rounds, bt->ls_plan_words, bt->ls_plan_init};
+    k_ls_sparse<<<grid, kLsThreads, kFastSmem, s>>>(A, S, bt->ls_list, (int)sparse.size(), direct ? 1 : 0,
+                                                    bt->ls_queue, bt->ls_scratch, slot,
+                                                    reinterpret_cast<const LsParams*>(bt->ls_params), bt->ls_pivot);
+    CFD_TRY_CUDA(cudaGetLastError());
+    bt->ctx->stats.launches++;
+    std::vector<int> piv(bt->nsys);
+    CFD_TRY_CUDA(cudaMemcpyAsync(piv.data(), bt->ls_pivot, bt->nsys * sizeof(int), cudaMemcpyDeviceToHost, s));
+    CFD_TRY_CUDA(cudaStreamSynchronize(s));
+    for (int sy : sparse)
+      if (piv[sy]) dense.push_back(sy);
+  }
+  int dmax = 1;
+  for (int sy : dense) dmax = std::max(dmax, bt->h_sys_row[sy + 1] - bt->h_sys_row[sy]);
+  return ls_dense_launch(bt, A, dense, dmax, direct, s);
+}
+
 template <bool REFINE>
 cfd_status ls_krylov_bucket(cfd_batch* bt, const LsArgs& A, int bkt, cudaStream_t s) {
   using T = typename std::conditional<REFINE, float, double>::type;
@@ -1148,12 +1398,7 @@ cfd_status cfd_batch_linear_system_solve(cfd_batch* bt, const cfd_ls_options* op
              bt->ls_method, bt->ls_path, bt->term, bt->iters, bt->resid};
     // direct systems: rows <= 256, the buckets below kBucketRows[2]
     std::vector<int> direct;
-    int dmax = 1;
-    for (int q = bt->bucket_begin[0]; q < bt->bucket_begin[2]; ++q) {
-      const int sy = bt->h_order[q];
-      direct.push_back(sy);
-      dmax = std::max(dmax, bt->h_sys_row[sy + 1] - bt->h_sys_row[sy]);
-    }
+    for (int q = bt->bucket_begin[0]; q < bt->bucket_begin[2]; ++q) direct.push_back(bt->h_order[q]);
     // Phase boundaries: start, after the direct solves, after the Krylov
     // launches, after the fallback (events released on every return).
     struct PhaseEvents {
@@ -1171,7 +1416,7 @@ cfd_status cfd_batch_linear_system_solve(cfd_batch* bt, const cfd_ls_options* op
       k_ls_detect<<<(int)((direct.size() + 7) / 8), 256, 0, s>>>(A, bt->ls_list, (int)direct.size(), fixed);
       CFD_TRY_CUDA(cudaGetLastError());
       ctx->stats.launches++;
-      CFD_TRY(ls_dense_launch(bt, A, direct, dmax, true, s));
+      CFD_TRY(ls_direct_launch(bt, A, direct, true, s));
     }
     CFD_TRY_CUDA(cudaEventRecord(ph.e[1], s));
     for (int k = kBuckets - 1; k >= 2; --k) {
@@ -1186,17 +1431,11 @@ cfd_status cfd_batch_linear_system_solve(cfd_batch* bt, const cfd_ls_options* op
     CFD_TRY_CUDA(cudaMemcpyAsync(path.data(), bt->ls_path, bt->nsys * sizeof(int), cudaMemcpyDeviceToHost, s));
     CFD_TRY_CUDA(cudaStreamSynchronize(s));
     CFD_TRY(check_device_flag(ctx));
-    // Krylov solves that were not kept: dense LU of the original system.
+    // Krylov solves that were not kept: a direct solve of the original system.
     std::vector<int> fallback;
-    int fmax = 1;
-    for (int q = bt->bucket_begin[2]; q < bt->nsys; ++q) {
-      const int sy = bt->h_order[q];
-      if (path[sy] == CFD_LS_PATH_KRYLOV_FALLBACK) {
-        fallback.push_back(sy);
-        fmax = std::max(fmax, bt->h_sys_row[sy + 1] - bt->h_sys_row[sy]);
-      }
-    }
-    CFD_TRY(ls_dense_launch(bt, A, fallback, fmax, false, s));
+    for (int q = bt->bucket_begin[2]; q < bt->nsys; ++q)
+      if (path[bt->h_order[q]] == CFD_LS_PATH_KRYLOV_FALLBACK) fallback.push_back(bt->h_order[q]);
+    CFD_TRY(ls_direct_launch(bt, A, fallback, false, s));
     CFD_TRY_CUDA(cudaEventRecord(ph.e[3], s));
     CFD_TRY_CUDA(cudaMemcpyAsync(x, bt->x, bt->rows * sizeof(double), outk, s));
     CFD_TRY_CUDA(cudaEventRecord(ctx->ev1, s));

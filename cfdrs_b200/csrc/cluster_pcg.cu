@@ -94,18 +94,14 @@ __device__ __forceinline__ uint32_t cl_map(uint32_t a, uint32_t rank) {
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(rank));
   return d;
 }
-// Loads and stores of the cluster's shared memory. Volatile keeps them between
-// the barriers that order them; consecutive loads still overlap.
-// The load only where `on` (a predicate, not a branch), else v as it is: the
+// A load of the cluster's shared memory (volatile keeps it between the barriers
+// that order it) only where `on` (a predicate, not a branch), else v as it is: the
 // cluster path is slow even for a CTA's own memory, so only lanes whose entry is
 // another CTA's take it.
 __device__ __forceinline__ void cl_ld_if(double& v, uint32_t a, bool on) {
   asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q ld.shared::cluster.f64 %0, [%1];\n}\n"
                : "+d"(v)
                : "r"(a), "r"((int)on));
-}
-__device__ __forceinline__ void cl_st(uint32_t a, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 __device__ __forceinline__ void cl_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

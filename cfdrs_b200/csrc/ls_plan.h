@@ -1,0 +1,55 @@
+// Elimination plans of the 1-D cascade's direct solves (batch_ls.cu).
+//
+// A pipe network is a tree with a few loops, so Gaussian elimination in an order
+// that takes nodes of low degree first creates almost no fill: nodes of degree
+// one and two leave a core of at most twice the loops, and eliminating up to
+// degree kLsPlanDegree shrinks it further. The plan is that order written out
+// for one sparsity pattern: rounds of independent nodes (no two adjacent), each a
+// list of divisions and a list of updates whose targets differ, and the core that
+// is left, which is solved densely. Diagonal pivots throughout; the kernel checks
+// every multiplier and hands a system that needs row exchanges to the dense path.
+//
+// Values live in numbered slots: the pattern's entries (closed under transposition,
+// the added ones zero), the fill, then one slot per row for the right-hand side,
+// which the solution replaces.
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+namespace cfd {
+
+constexpr int kLsPlanDegree = 4;
+constexpr int kLsPlanMaxSlots = 20000;
+
+// Words (uint16) of a round, from `at`:
+//   divisions: nl pairs (l, d): v[l] /= v[d]
+//   targets:   nt triples (t, first, count): v[t] -= sum of count products,
+//              products being pairs (i, j) from word pairs + 2 first
+//   solutions: nx quadruples (b, d, first, count): v[b] = (v[b] - sum of count
+//              products) / v[d], products from word xpairs + 2 first
+struct LsRound {
+  int32_t at_l, nl, at_t, nt, pairs, at_x, nx, xpairs;
+};
+
+struct LsPlanHead {
+  int32_t ok;             // 0: no plan (the dense path)
+  int32_t slots, b0;      // slots in all, first right-hand-side slot
+  int32_t round0, rounds; // this system's rounds
+  int32_t core, at_core;  // core nodes: word at_core + k
+  int32_t entries, at_entries;  // core entries: triples (slot, row, col)
+  int32_t pad;
+  int64_t words;          // this system's first word
+  int64_t init;           // slot of every stored entry, first word (the batch's entry order)
+};
+
+// The plan of one square pattern (rows rp[0..n], local columns); words and
+// rounds are appended, head.words / head.init left to the caller.
+struct LsPlanOne {
+  LsPlanHead head{};
+  std::vector<uint16_t> words, init;
+  std::vector<LsRound> rounds;
+};
+void ls_plan_build(int n, const int* rp, const int* col, LsPlanOne& out);
+
+}  // namespace cfd
