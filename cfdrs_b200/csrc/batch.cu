@@ -1226,6 +1226,9 @@ cfd_status cfd_batch_destroy(cfd_batch* bt) {
                   (void*)bt->ls_pivot, (void*)bt->ls_plan_heads, (void*)bt->ls_plan_rounds,
                   (void*)bt->ls_plan_words, (void*)bt->ls_plan_init})
     if (p) cudaFree(p);
+  if (bt->ls_branch) cudaStreamDestroy(bt->ls_branch);
+  if (bt->ls_fork) cudaEventDestroy(bt->ls_fork);
+  if (bt->ls_join) cudaEventDestroy(bt->ls_join);
   if (bt->h_params) cudaFreeHost(bt->h_params);
   network_plan_free(bt->net);
   delete bt;

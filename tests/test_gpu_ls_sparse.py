@@ -109,3 +109,30 @@ def test_singular_system_fails_alone(cuda):
     x, rep = nb.solve_linear_systems(np.ones(600), tolerance=1e-10, max_iterations=1, method=LS_BICGSTAB)
     assert LS_PATHS[rep.path[0]] == "krylov_fallback" and LS_PATHS[rep.path[1]] == "failed"
     assert np.all(np.isfinite(nb.split(x)[0]))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_refine"])
+@pytest.mark.parametrize("method", ["detect", "cg"])
+def test_krylov_rows_in_registers_match_shared_memory_vectors(cuda, precision, method):
+    """The register form of the Krylov kernel (at most 8 rows a thread, 256
+    threads) forms every sum in the order of the shared-memory form: with the same
+    width in both buckets the outcome is the same bits, whichever form the wider
+    bucket's row count selects."""
+    import cfdrs_b200 as cf
+    from cfdrs_b200 import problems as P
+    from cfdrs_b200.batch import LS_CG, LS_DETECT, NetworkBatch
+    rng = np.random.default_rng(9)
+    prec = cf.Precision.FP64 if precision == "fp64" else cf.Precision.FP32_REFINE
+    meth = LS_DETECT if method == "detect" else LS_CG
+    small = [P.random_network(n, rng) for n in (257, 300, 511, 512)]
+    got = []
+    for extra in (None, 513):  # 64 threads: 512 rows are 8 a thread, 513 are 9 (shared memory)
+        systems = small + ([P.random_network(extra, np.random.default_rng(1))] if extra else [])
+        nb = NetworkBatch([A for A, _ in systems])
+        nb.set_config([32, 64, 64, 256], [1, 1, 1, 1], prec)
+        x, rep = nb.solve_linear_systems(np.concatenate([b for _, b in systems]), tolerance=1e-10, method=meth,
+                                         precision=prec)
+        rows = sum(A.nrows for A, _ in small)
+        got.append((x[:rows], rep.iterations[:4], rep.termination[:4], rep.path[:4]))
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
