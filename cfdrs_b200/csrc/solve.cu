@@ -704,6 +704,27 @@ struct Launcher {
   static bool dia_ready(const DevMat& m) {
     return m.dia && (sizeof(VT) == 8 ? m.dia64 != nullptr : (m.dia32 != nullptr && m.v32 != nullptr));
   }
+  // The direct kernel takes the operators of default choice that are small
+  // enough: one thread or row group per row, no persistence.
+  template <typename VT, typename XT, bool OFF, class Epi>
+  cfd_status direct_launch(const DevMat& m, const XT* x, Epi epi) {
+    const int64_t threads = m.nrows * (int64_t)m.tpr;
+    const int grid = (int)((threads + kThreads - 1) / kThreads);
+    launch(k_spmv_direct<VT, XT, OFF, Epi>, grid, kThreads, 0, mat_view<VT>(m), (int)m.nrows, x, epi);
+    return CFD_OK;
+  }
+  // Values and columns of at most 16 MB (a launch of a few microseconds, where
+  // the latency chain counts), and with a reduction at most one slot per CTA. Both
+  // sides measured by moving the limit: 512^2 adjoint 8.03 ms without the kernel,
+  // 7.23 / 7.10 / 7.00 / 6.95 ms up to 0.1 / 0.3 / 0.8 / 3 M FP32 entries; 96^3 FP64
+  // 3.28 ms without, 3.24 ms to 0.8 M, 3.27 to 3 M, 3.33 to 12 M; 192^3 FP32 14.89 ms
+  // without, 14.70 to 3 M, 15.07 to 12 M.
+  template <typename VT>
+  static bool direct_fits(const DevMat& m, int p, int nred) {
+    const int64_t grid = (m.nrows * (int64_t)m.tpr + kThreads - 1) / kThreads;
+    return m.path[p] == CFD_PATH_AUTO && m.nnz * (int64_t)(sizeof(VT) + 4) <= (int64_t)16 << 20 &&
+           (nred == 0 || grid <= kVecGrid);
+  }
   static constexpr int kPathTimed = -2, kPathSplit = 0, kPathRecord = 1, kPathXs = 2, kPathSliced = 3,
                        kPathDiag = 4;
   template <typename VT, typename XT, bool OFF, class Epi>
@@ -726,6 +747,10 @@ struct Launcher {
         CFD_TRY((dia_launch<VT, OFF, Epi>(m, x, epi)));
         return finish_spmv<VT, XT>(m);
       }
+    }
+    if (direct_fits<VT>(m, p, Epi::NRED)) {
+      CFD_TRY((direct_launch<VT, XT, OFF, Epi>(m, x, epi)));
+      return finish_spmv<VT, XT>(m);
     }
     if (path == kPathDiag) path = m.all_compressed ? kPathRecord : kPathSplit;
     if constexpr (std::is_same<VT, XT>::value) {
