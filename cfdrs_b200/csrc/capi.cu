@@ -364,6 +364,7 @@ void amg_free_device(cfd_amg* amg) {
   }
   amg->dev.clear();
   dfree(amg->coarse_inv);
+  dfree(amg->coarse_spare);
   dfree(amg->coarse_inv32);
   amg->have32 = false;
 }
