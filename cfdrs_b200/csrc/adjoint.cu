@@ -171,8 +171,10 @@ cfd_status cfd_csr_set_values_device(cfd_csr* a, const double* val_dev) {
   }
   a->dev.sl_stale = true;
   a->dev.dia_stale = true;
-  // The host copy feeds AMG setup (the Galerkin recompute reads the device values).
-  CFD_TRY_CUDA(cudaMemcpyAsync(a->host.v.data(), val_dev, nnz * sizeof(double), cudaMemcpyDeviceToHost, s));
+  // The host copy (AMG and saddle-point setup, diagonals, the transpose) is
+  // brought up to date by its next reader: copying 10 MB back here at every new
+  // set of values was 0.6 of a 512^2 adjoint update's 7.0 ms, which reads none of it.
+  a->host_stale = true;
   CFD_TRY_CUDA(cudaStreamSynchronize(s));
   a->values_version++;
   a->simple_stale = a->simple_nv >= 0;

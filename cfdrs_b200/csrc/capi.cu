@@ -305,8 +305,18 @@ cfd_status check_device_flag(cfd_context* ctx) {
 // Diagonal of A (FP64/FP32) and the DiagJacobi inverse: 1/a_ii, or 1 where
 // |a_ii| <= f64::EPSILON (linear_system.rs:286-295); a non-finite diagonal
 // entry makes the Jacobi preconditioner unavailable (linear_system.rs:281-285).
+cfd_status csr_sync_host(cfd_csr* a) {
+  if (!a->host_stale) return CFD_OK;
+  cudaStream_t s = a->ctx->stream;
+  CFD_TRY_CUDA(cudaMemcpyAsync(a->host.v.data(), a->dev.v64, a->dev.nnz * sizeof(double), cudaMemcpyDeviceToHost, s));
+  CFD_TRY_CUDA(cudaStreamSynchronize(s));
+  a->host_stale = false;
+  return CFD_OK;
+}
+
 cfd_status ensure_diagonals(cfd_csr* a) {
   if (a->diag64) return CFD_OK;
+  CFD_TRY(csr_sync_host(a));
   const HostCsr& h = a->host;
   const int64_t n = h.nrows;
   std::vector<double> d(n, 0.0), inv(n, 1.0);
@@ -654,6 +664,7 @@ cfd_status cfd_csr_update_values(cfd_csr* a, const double* val) {
     // only once the device copy and the FP32 cast have succeeded.
     CFD_TRY(devmat_update_values(a->dev, val, a->host.nnz(), false, a->ctx->stream));
     std::copy(val, val + a->host.nnz(), a->host.v.begin());
+    a->host_stale = false;
     a->values_version++;
     a->simple_stale = a->simple_nv >= 0;
     a->cblock_stale = a->cblock_nv >= 0;
@@ -850,6 +861,7 @@ cfd_status cfd_amg_setup(cfd_csr* a, const cfd_amg_config* cfg, cfd_amg** out) {
     }
     std::lock_guard<std::mutex> g(a->ctx->mu);
     CFD_TRY_CUDA(cudaSetDevice(a->ctx->device));
+    CFD_TRY(csr_sync_host(a));
     auto t0 = std::chrono::steady_clock::now();
     cfd_amg* amg = new cfd_amg;
     OnUnwind release([&] {
@@ -1046,6 +1058,7 @@ static cfd_status csr_transposed(cfd_csr* a, cfd_csr** out) {
     *out = a->tr;
     return CFD_OK;
   }
+  CFD_TRY(csr_sync_host(a));
   const HostCsr& h = a->host;
   HostCsr T;
   T.nrows = h.ncols;

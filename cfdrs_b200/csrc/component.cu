@@ -126,6 +126,7 @@ void component_free(ComponentDev* C) {
 // inverse limit or a singular block (the reference's constructor Errs).
 cfd_status component_build(cfd_csr* a, int64_t nv, double pivot_tolerance, ComponentDev** out) {
   *out = nullptr;
+  CFD_TRY(csr_sync_host(a));
   const HostCsr& h = a->host;
   const int64_t n = h.nrows;
   if (h.ncols != n || nv <= 0 || nv > n || nv % 3 != 0) {

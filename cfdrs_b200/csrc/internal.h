@@ -347,6 +347,7 @@ struct cfd_csr {
   // Value updates so far, and the transpose (cfd_adjoint with transpose != 0),
   // formed from the values of update tr_version.
   uint64_t values_version = 0;
+  bool host_stale = false;  // host.v lags the device values (csr_sync_host)
   cfd_csr* tr = nullptr;
   uint64_t tr_version = 0;
   // Boundary entries of the fullest row block of the grid CG (grid_pcg.cu), -1
@@ -360,6 +361,9 @@ cfd_status ensure_partials(cfd_context* ctx, int blocks);
 // as CFD_ERR_TIMEOUT and the flag and reduction ticket are reset.
 cfd_status check_device_flag(cfd_context* ctx);
 cfd_status ensure_diagonals(cfd_csr* a);
+// Brings host.v up to date with values set on the device; every reader of
+// host.v calls it first (with the context's lock held).
+cfd_status csr_sync_host(cfd_csr* a);
 // g_e = -scale * lambda[row(e)] * x[col(e)] over A's pattern, on the context stream.
 cfd_status pattern_outer_launch(cfd_csr* a, const double* lambda, const double* x, double scale, double* g);
 // Whole CG / Jacobi-PCG solve in one thread-block cluster (cluster_pcg.cu):

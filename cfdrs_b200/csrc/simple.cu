@@ -189,6 +189,7 @@ cfd_status simple_ensure(cfd_csr* a) {
     return CFD_ERR_STATE;
   }
   if (a->simple && !a->simple_stale) return CFD_OK;
+  CFD_TRY(csr_sync_host(a));
   SimpleHost S;
   CFD_TRY(simple_build(a->host, a->simple_nv, S));
   SimpleDev* D = new SimpleDev;
@@ -256,6 +257,7 @@ cfd_status cfd_saddle_setup(cfd_csr* a, int64_t n_velocity) {
     if (!a) return CFD_ERR_STATE;
     std::lock_guard<std::mutex> g(a->ctx->mu);
     CFD_TRY_CUDA(cudaSetDevice(a->ctx->device));
+    CFD_TRY(csr_sync_host(a));
     SimpleHost S;
     CFD_TRY(simple_build(a->host, n_velocity, S));
     a->simple_nv = n_velocity;

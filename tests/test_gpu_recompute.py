@@ -194,3 +194,61 @@ def test_recompute_leaves_other_matrices_alone(cuda):
     rep = cf.cg_preconditioned(A1, b1, amg, x, cf.IterativeSolverConfig(0.0, 1e-10, 1000))
     assert rep.termination == cf.Termination.CONVERGED
     assert np.linalg.norm(A1.to_scipy() @ x - b1) <= 1e-9 * np.linalg.norm(b1)
+
+
+def gauss_jordan(D):
+    """The host dense_inverse's operations in its order (products rounded before
+    the subtraction), by rows."""
+    n = D.shape[0]
+    m, inv = D.copy(), np.eye(n)
+    for c in range(n):
+        p = c + int(np.argmax(np.abs(m[c:, c])))
+        m[[c, p]] = m[[p, c]]
+        inv[[c, p]] = inv[[p, c]]
+        d = 1.0 / m[c, c]
+        m[c] *= d
+        inv[c] *= d
+        f = m[:, c].copy()
+        f[c] = 0.0
+        for r in np.flatnonzero(f):
+            m[r] -= f[r] * m[c]
+            inv[r] -= f[r] * inv[c]
+    return inv
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 100, 159, 160, 161])
+def test_small_dense_inverse_is_the_host_elimination(cuda, n):
+    """Up to 160 rows the coarsest inverse is formed in one CTA, beyond in the
+    cooperative launch; both are the host elimination bit for bit. Random signs
+    force row exchanges; some columns hold equal magnitudes (first row wins)."""
+    import cfdrs_b200 as cf
+    rng = np.random.default_rng(n)
+    D = rng.choice([-1.0, -0.5, 0.0, 0.5, 1.0], (n, n)) + np.eye(n) * rng.choice([-3.0, 3.0], n)
+    amg = cf.AlgebraicMultigrid(from_scipy(sp.csr_matrix(D)),
+                                cf.AMGConfig(max_levels=1, coarse_solve=cf.CoarseSolve.DENSE))
+    got = np.stack([np.asarray(amg.apply_to(e)) for e in np.eye(n)], axis=1)
+    np.testing.assert_array_equal(got, gauss_jordan(D) + 0.0)  # + 0.0: a zero's sign is not kept
+
+
+def test_device_values_reach_every_host_reader(cuda):
+    """Values set on the device are what a later Jacobi diagonal, AMG setup and
+    saddle split see, although the host copy is brought up to date only there."""
+    import cfdrs_b200 as cf
+    from cfdrs_b200 import adjoint, problems as P
+    torch = cuda
+    A, b = P.poisson_2d_dirichlet(20, 17, seed=2)
+    bd = torch.as_tensor(b, device="cuda")
+    rng = np.random.default_rng(5)
+    for kind in ("jacobi", "amg"):
+        solver = adjoint.SparseSolver(A, preconditioner=kind, precision=cf.Precision.FP64)
+        for k in range(3):
+            s = np.sqrt(rng.uniform(0.5, 2.0, A.nrows))
+            M = A.to_scipy().multiply(s[:, None]).multiply(s[None, :]).tocsr()
+            M.sort_indices()
+            solver.set_values(torch.as_tensor(M.data, device="cuda"), rebuild=k == 2)
+            x = solver.solve(bd).cpu().numpy()
+            assert np.linalg.norm(M @ x - b) <= 1.1e-10 * np.linalg.norm(b)
+            if kind == "amg" and k == 2:  # the rebuilt hierarchy is a fresh setup's
+                fresh = cf.AlgebraicMultigrid(from_scipy(M), solver.amg_config)
+                last = fresh.num_levels - 1
+                np.testing.assert_array_equal(solver.amg.level(last).val, fresh.level(last).val)
