@@ -1171,6 +1171,12 @@ int gmres_width(int64_t requested) {
   return w;
 }
 
+// Steps until a residual that falls by `rate` a step passes the threshold.
+static double gmres_steps_left(double rn, const DevState& h, double rate) {
+  if (!(h.threshold > 0.0) || !(rn > h.threshold)) return 1.0;
+  return std::max(1.0, std::ceil(std::log(h.threshold / rn) / std::log(rate)));
+}
+
 // Restarted GMRES(m) with right preconditioning. Expects the state's start
 // (rnorm0, threshold, done, iter) set, r = b - A x and b the right-hand side.
 // One host poll per restart cycle; the steps of a cycle after it ended are
@@ -1225,7 +1231,18 @@ static cfd_status gmres_loop(Launcher& lc, cfd_csr* a, cfd_amg* amg, KrylovBufs<
     return v;
   };
   int64_t cycles = 0;
+  // Steps launched after a cycle has ended return at once but cost a launch each
+  // (nine to fifty kernels a step): the host looks at the state where the
+  // residual's rate says the cycle should end, and stops launching once it has.
+  // A restart of 32 that converged in 17 steps ran 15 for nothing, 2.75 ms against
+  // 2.02 ms on the 11^3 Stokes system. A rate that reaches past the restart costs
+  // no look.
+  double rate = 0.0, rn_cycle = 0.0;
   for (;;) {
+    int look = 8;
+    if (cycles > 0) look = rate > 0.0 && rate < 1.0 ? (int)std::min(1e6, gmres_steps_left(rn_cycle, *pl.host, rate)) : m;
+    int last_look = 0;
+    double last_rn = rn_cycle;
     // cycle start: beta = ||r||, v_0 = r / beta
     k_gmres_begin<<<1, 1, 0, lc.s>>>(G, st);
     CFD_TRY(dots(B.r, 1, B.r, G.g, 1, done));
@@ -1245,6 +1262,16 @@ static cfd_status gmres_loop(Launcher& lc, cfd_csr* a, cfd_amg* amg, KrylovBufs<
       CFD_TRY(lc.vec(n, k_scale_div<XT>, (const XT*)w, w, (const double*)(hc + j + 1), ended));
       k_gmres_rot<<<1, 1, 0, lc.s>>>(G, j, st);
       CFD_TRY(lc.check());
+      if (j + 1 == look && j + 1 < m) {
+        CFD_TRY(pl.poll());
+        const DevState& h = *pl.host;
+        if (h.done || !(h.rnorm > h.threshold) || h.iter >= h.max_iter) break;
+        const double from = last_rn > 0.0 ? last_rn : h.rnorm0;
+        rate = from > 0.0 ? std::pow(h.rnorm / from, 1.0 / (double)(j + 1 - last_look)) : 0.0;
+        last_look = j + 1;
+        last_rn = h.rnorm;
+        look = rate > 0.0 && rate < 1.0 ? j + 1 + (int)std::min(1e6, gmres_steps_left(h.rnorm, h, rate)) : m;
+      }
     }
     // x += M^-1 (V y); r = b - A x; the true residual decides
     k_gmres_lsq<<<1, 1, 0, lc.s>>>(G, done);
@@ -1257,6 +1284,7 @@ static cfd_status gmres_loop(Launcher& lc, cfd_csr* a, cfd_amg* amg, KrylovBufs<
     CFD_TRY(lc.check());
     CFD_TRY(pl.poll());
     if (pl.host->done) break;
+    rn_cycle = pl.host->rnorm;
     if (++cycles > pl.host->max_iter + 2) {
       set_error("GMRES did not terminate within its iteration budget");
       return CFD_ERR_TIMEOUT;
