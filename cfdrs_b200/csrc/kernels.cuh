@@ -1076,6 +1076,75 @@ struct DiaVecN<float, 2> {
   }
 };
 
+// Row of a dense matrix times a vector in FP64, for a grid of dense_grid(rows, W)
+// CTAs of kThreads: returns the row in the thread that holds its sum, -1 elsewhere.
+// What bounds it: the matrix (33 MB for 2876 FP32 rows) comes from L2, so enough
+// of it has to be in flight: a row is shared by W warps, each lane with four 16-byte
+// loads of it and the vector's matching ones, where rows and vector start on 16-byte
+// boundaries (an n divisible by the vector); scalar loads otherwise. W is 4 while
+// all rows' warps are resident at once and 2 beyond (dense_wide); time in us of W
+// 1 / 2 / 4, and of one warp a row with scalar loads:
+//   1402 rows FP64           11.5 / 9.4 / 7.1    10.7
+//   2876 rows FP32           10.8 / 8.8 / 11.1   11.3
+//   3 x 1210 rows FP64        7.7 / 6.4 / 9.1    11.1 (three launches)
+inline bool dense_wide(int64_t rows) { return rows <= 2048; }
+inline int dense_grid(int n, int w) { return (n + kThreads / 32 / w - 1) / (kThreads / 32 / w); }
+
+template <int W, typename IT, typename XT>
+__device__ __forceinline__ int dense_row_dot(int n, const IT* __restrict__ m, const XT* __restrict__ b, double& sum) {
+  __shared__ double part[kThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = warp % W;
+  const int row = blockIdx.x * (kThreads / 32 / W) + warp / W;
+  double s = 0.0;
+  if (row < n) {
+    const IT* a = m + (size_t)row * n;
+    constexpr int V = DiaVec<IT>::V, Q = 4, T = 32 * W;
+    constexpr int VB = V * sizeof(XT) > 16 ? V / 2 : V;  // FP64 vector of an FP32 matrix: two loads
+    using VecB = DiaVecN<XT, VB>;
+    const int t = w * 32 + lane;
+    if (n % V == 0 && ((uintptr_t)m & (V * sizeof(IT) - 1)) == 0 && ((uintptr_t)b & (VB * sizeof(XT) - 1)) == 0) {
+      for (int k0 = t * V; k0 < n; k0 += Q * T * V) {
+        IT av[Q][V];
+        XT bv[Q][V];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const int k = k0 + q * T * V;
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            av[q][v] = IT(0);
+            bv[q][v] = XT(0);
+          }
+          if (k < n) {
+            DiaVec<IT>::unpack(__ldg(reinterpret_cast<const typename DiaVec<IT>::type*>(a + k)), av[q]);
+#pragma unroll
+            for (int h = 0; h < V; h += VB) {
+              XT o[VB];
+              VecB::unpack(*reinterpret_cast<const typename VecB::type*>(b + k + h), o);
+#pragma unroll
+              for (int v = 0; v < VB; ++v) bv[q][h + v] = o[v];
+            }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+          for (int v = 0; v < V; ++v) s += (double)av[q][v] * (double)bv[q][v];
+      }
+    } else {
+#pragma unroll 8
+      for (int k = t; k < n; k += T) s += (double)a[k] * (double)b[k];
+    }
+    s = warp_sum(s);
+  }
+  if (lane == 0) part[warp] = s;
+  __syncthreads();
+  if (w != 0 || lane != 0 || row >= n) return -1;
+  sum = 0.0;
+#pragma unroll
+  for (int q = 0; q < W; ++q) sum += part[warp + q];
+  return row;
+}
+
 // x operand of the diagonal kernels (a stored vector; the kernels take it as
 // a source object so a fused producer of x can take its place).
 template <typename VT>
