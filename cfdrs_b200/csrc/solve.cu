@@ -415,37 +415,178 @@ __global__ void k_gmres_begin(GmresDev G, const DevState* st) {
   for (int k = 1; k <= G.m; ++k) G.g[k] = 0.0;
 }
 
-// Step j: second projection pass added to the column, earlier rotations
+// Step j on the column h (projections, then the norm h[j + 1]): earlier rotations
 // applied, the new rotation formed, the implicit residual |g_{j+1}| tested.
-__global__ void k_gmres_rot(GmresDev G, int j, DevState* st) {
-  if (G.flags[1]) return;
-  const int m = G.m;
-  double* h = G.H + (size_t)j * (m + 1);
-  for (int q = 0; q <= j; ++q) h[q] += G.h[q];
+__device__ __forceinline__ void gmres_rotation(const GmresDev& G, int j, DevState* st, double* h, const double* cs,
+                                               const double* sn) {
   const double hn = h[j + 1];
   for (int q = 0; q < j; ++q) {
-    const double t = G.cs[q] * h[q] + G.sn[q] * h[q + 1];
-    h[q + 1] = -G.sn[q] * h[q] + G.cs[q] * h[q + 1];
+    const double t = cs[q] * h[q] + sn[q] * h[q + 1];
+    h[q + 1] = -sn[q] * h[q] + cs[q] * h[q + 1];
     h[q] = t;
   }
   const double d = hypot(h[j], h[j + 1]);
-  G.cs[j] = d > 0.0 ? h[j] / d : 1.0;
-  G.sn[j] = d > 0.0 ? h[j + 1] / d : 0.0;
+  const double c = d > 0.0 ? h[j] / d : 1.0, s = d > 0.0 ? h[j + 1] / d : 0.0, gj = G.g[j];
+  G.cs[j] = c;
+  G.sn[j] = s;
   h[j] = d;
   h[j + 1] = 0.0;
-  G.g[j + 1] = -G.sn[j] * G.g[j];
-  G.g[j] = G.cs[j] * G.g[j];
+  G.g[j + 1] = -s * gj;
+  G.g[j] = c * gj;
   st->iter += 1;
-  const double res = fabs(G.g[j + 1]);
+  const double res = fabs(s * gj);
   st->rnorm = res;
   G.flags[0] = j + 1;
   if (!isfinite(res)) {
     G.flags[1] = 1;
     st->term = CFD_TERM_BREAKDOWN;
     st->done = 1;
-  } else if (res <= st->threshold || st->iter >= st->max_iter || hn == 0.0 || j + 1 == m) {
+  } else if (res <= st->threshold || st->iter >= st->max_iter || hn == 0.0 || j + 1 == G.m) {
     G.flags[1] = 1;
   }
+}
+
+// The second projection pass added to the column, then the rotation.
+__global__ void k_gmres_rot(GmresDev G, int j, DevState* st) {
+  if (G.flags[1]) return;
+  double* h = G.H + (size_t)j * (G.m + 1);
+  for (int q = 0; q <= j; ++q) h[q] += G.h[q];
+  gmres_rotation(G, j, st, h, G.cs, G.sn);
+}
+
+// A whole Arnoldi step of a small system (both projection passes, the norm, the
+// scaling and the rotation) in one cluster: V_{j+1} = w on entry. Each CTA holds its
+// rows of w in shared memory; warps form the CTA's shares of V_k . w, which meet in
+// distributed shared memory (pulled after a cluster barrier and summed in rank
+// order by every CTA, so all hold the same bits). The separate kernels are
+// eight launches, half of them a reduction over a few thousand rows; here the
+// bound is latency (three barriers with their pulls, two reads of V from L2 a
+// pass) and, as n nv grows, what eight SMs read. Time of a step in us at 1 / 5 / 9 / 17
+// columns, separate kernels and this one:
+//    4961 rows   37 / 31 / 40 / 51    19 / 12 / 14 / 17
+//   15616 rows   40 / 34 / 45 / 61    24 / 19 / 26 / 36
+// and 57 us against 48 at 30800 rows and 9 columns (512 threads, 4096 rows a CTA): orth_fits. With
+// 512 threads 4961 rows took 24 us at 17 columns, with 16 loads in flight a lane 21.
+constexpr int kOrthCtas = 8;  // the portable cluster size
+constexpr int kOrthThreads = 1024;
+constexpr int kOrthWarps = kOrthThreads / 32;
+constexpr int kOrthRows = 2048;   // rows of a CTA
+constexpr int kOrthWidth = 256;   // largest restart width (gmres_width)
+constexpr int kOrthLoads = 8;     // loads of a lane in flight
+inline bool orth_fits(int64_t n, int nv) { return n <= kOrthCtas * kOrthRows && nv <= kOrthWidth && n * nv <= 1 << 20; }
+
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  cluster_arrive();
+  cluster_wait();
+}
+__device__ __forceinline__ double orth_pull(const double* p, uint32_t rank) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+  double v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(r) : "memory");
+  return v;
+}
+__device__ __forceinline__ double orth_sum8(double v) {
+#pragma unroll
+  for (int o = 1; o < kOrthCtas; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+template <typename XT>
+__global__ void __cluster_dims__(kOrthCtas, 1, 1) __launch_bounds__(kOrthThreads)
+    k_gmres_orth(int64_t n, XT* __restrict__ V, int j, GmresDev G, DevState* st) {
+  __shared__ double w[kOrthRows];
+  __shared__ double part[2][kOrthWidth], h[2][kOrthWidth + 1], cs[kOrthWidth], sn[kOrthWidth], share[kOrthWarps], nrm;
+  pdl_enter();
+  if (G.flags[1]) return;  // written at the end of a step, after barriers every CTA has passed
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nv = j + 1;
+  const int rank = (int)blockIdx.x;  // one cluster
+  const int64_t rpc = (n + kOrthCtas - 1) / kOrthCtas, r0 = rank * rpc;
+  const int nr = (int)(r0 >= n ? 0 : (n - r0 < rpc ? n - r0 : rpc));
+  const XT* Vr = V + r0;
+  XT* wg = V + (size_t)nv * n + r0;
+  for (int i = tid; i < nr; i += kOrthThreads) w[i] = (double)wg[i];
+  if (rank == 0)
+    for (int q = tid; q < j; q += kOrthThreads) {
+      cs[q] = G.cs[q];
+      sn[q] = G.sn[q];
+    }
+  __syncthreads();
+  int sp = 0;
+  while (sp < 3 && nv << (sp + 1) <= kOrthWarps) ++sp;
+  double nsq = 0.0;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    // few columns: 2^sp warps a column, their shares added in order
+    for (int k = warp >> sp; k < nv; k += kOrthWarps >> sp) {
+      const XT* vk = Vr + (size_t)k * n;
+      const int t = (warp & ((1 << sp) - 1)) * 32 + lane, step = 32 << sp;
+      double s = 0.0;
+      for (int i0 = t; i0 < nr; i0 += step * kOrthLoads) {
+        XT x[kOrthLoads];
+#pragma unroll
+        for (int q = 0; q < kOrthLoads; ++q) x[q] = i0 + step * q < nr ? vk[i0 + step * q] : XT(0);
+#pragma unroll
+        for (int q = 0; q < kOrthLoads; ++q)
+          if (i0 + step * q < nr) s += (double)x[q] * w[i0 + step * q];
+      }
+      s = warp_sum(s);
+      if (lane == 0) (sp ? share[warp] : part[pass][k]) = s;
+    }
+    if (sp) {
+      __syncthreads();
+      if (tid < nv) {
+        double s = 0.0;
+        for (int q = 0; q < 1 << sp; ++q) s += share[(tid << sp) + q];
+        part[pass][tid] = s;
+      }
+    }
+    cluster_barrier();
+    for (int k0 = 0; k0 < nv; k0 += kOrthThreads / kOrthCtas) {
+      const int k = k0 + tid / kOrthCtas, src = tid % kOrthCtas;
+      const double s = orth_sum8(k < nv ? orth_pull(&part[pass][k], src) : 0.0);
+      if (k < nv && src == 0) h[pass][k] = s;
+    }
+    __syncthreads();
+    for (int i = tid; i < nr; i += kOrthThreads) {
+      double s = 0.0;
+      for (int k0 = 0; k0 < nv; k0 += kOrthLoads) {
+        XT x[kOrthLoads];
+#pragma unroll
+        for (int q = 0; q < kOrthLoads; ++q) x[q] = k0 + q < nv ? Vr[(size_t)(k0 + q) * n + i] : XT(0);
+#pragma unroll
+        for (int q = 0; q < kOrthLoads; ++q)
+          if (k0 + q < nv) s += h[pass][k0 + q] * (double)x[q];
+      }
+      const double wi = (double)(XT)(w[i] - s);
+      w[i] = wi;
+      if (pass == 1) nsq += wi * wi;
+    }
+    __syncthreads();
+  }
+  nsq = block_sum(nsq);
+  if (tid == 0) nrm = nsq;
+  cluster_barrier();
+  const double hn = sqrt(orth_sum8(orth_pull(&nrm, lane % kOrthCtas)));
+  cluster_arrive();  // this CTA has read its last of the others' shared memory
+  for (int i = tid; i < nr; i += kOrthThreads) wg[i] = (XT)(hn != 0.0 ? w[i] / hn : w[i]);
+  if (rank == 0 && warp == 0) {
+    for (int q = lane; q < nv; q += 32) h[0][q] += h[1][q];
+    if (lane == 0) h[0][nv] = hn;
+    __syncwarp();
+    if (lane == 0) gmres_rotation(G, j, st, h[0], cs, sn);
+    __syncwarp();
+    for (int q = lane; q <= nv; q += 32) G.H[(size_t)j * (G.m + 1) + q] = h[0][q];
+  }
+  cluster_wait();
 }
 
 // y = R^-1 g on the cycle's columns (back substitution).
@@ -1251,13 +1392,18 @@ static cfd_status gmres_loop(Launcher& lc, cfd_csr* a, cfd_amg* amg, KrylovBufs<
       const XT* z = precond(vj, B.z, ended);
       if (!z) return CFD_ERR_CUDA;
       CFD_TRY(lc.spmv<XT, XT, false>(a->dev, z, EpiStore<XT>{w, ended, {}}));
-      CFD_TRY(dots(V, j + 1, w, hc, 0, ended));
-      CFD_TRY(lc.vec(n, k_gemv_sub<XT>, (const XT*)V, n, j + 1, (const double*)hc, w, ended));
-      CFD_TRY(dots(V, j + 1, w, G.h, 0, ended));
-      CFD_TRY(lc.vec(n, k_gemv_sub<XT>, (const XT*)V, n, j + 1, (const double*)G.h, w, ended));
-      CFD_TRY(dots(w, 1, w, hc + j + 1, 1, ended));
-      CFD_TRY(lc.vec(n, k_scale_div<XT>, (const XT*)w, w, (const double*)(hc + j + 1), ended));
-      k_gmres_rot<<<1, 1, 0, lc.s>>>(G, j, st);
+      if (lc.ctx->cluster_solve && orth_fits(n, j + 1)) {
+        lc.launch(k_gmres_orth<XT>, kOrthCtas, kOrthThreads, 0, n, V, j, G, st);
+        lc.ctx->stats.launches++;
+      } else {
+        CFD_TRY(dots(V, j + 1, w, hc, 0, ended));
+        CFD_TRY(lc.vec(n, k_gemv_sub<XT>, (const XT*)V, n, j + 1, (const double*)hc, w, ended));
+        CFD_TRY(dots(V, j + 1, w, G.h, 0, ended));
+        CFD_TRY(lc.vec(n, k_gemv_sub<XT>, (const XT*)V, n, j + 1, (const double*)G.h, w, ended));
+        CFD_TRY(dots(w, 1, w, hc + j + 1, 1, ended));
+        CFD_TRY(lc.vec(n, k_scale_div<XT>, (const XT*)w, w, (const double*)(hc + j + 1), ended));
+        k_gmres_rot<<<1, 1, 0, lc.s>>>(G, j, st);
+      }
       CFD_TRY(lc.check());
       if (j + 1 == look && j + 1 < m) {
         CFD_TRY(pl.poll());
