@@ -646,9 +646,9 @@ def run_plain(args, world, rank, local):
             "roofline": ({"bound": "latency", "achieved": None, "peak": peak, "unit": "GB/s", "frac": None,
                           "traffic": None, "peak_kind": peak_kind,
                           "kernel": "k_cluster_pcg: the whole Jacobi-PCG solve in one thread-block cluster "
-                                    f"launch, {1e3 * ms / max(rep.iterations, 1):.2f} us per iteration (three "
-                                    "cluster barriers and two cluster reductions each; the system, 1.3 MB, "
-                                    "lives in distributed shared memory)"}
+                                    f"launch, {1e3 * ms / max(rep.iterations, 1):.2f} us per iteration (two "
+                                    "cluster barriers and two cluster reductions each; the rows live in registers, "
+                                    "the vectors in distributed shared memory)"}
                          if args.workload == "c1" and launches <= 2 else
                          {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
                           "traffic": None, "peak_kind": peak_kind,

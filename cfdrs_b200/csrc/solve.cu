@@ -300,6 +300,7 @@ __global__ void __launch_bounds__(kThreads) k_axpy_state(int64_t n, XT* __restri
 // (k_mdot per-CTA partials, k_mdot_finish in fixed order), the subtraction one
 // pass (k_gemv_sub); the Hessenberg column, the Givens rotations and the
 // implicit residual live on the device (k_gmres_rot, one thread).
+// Small systems take the whole step in one cluster launch (k_gmres_orth).
 constexpr int kGmresGrid = 148 * 2;
 constexpr int kDotTile = 8;
 
@@ -1317,8 +1318,8 @@ static double gmres_steps_left(double rn, const DevState& h, double rate) {
 
 // Restarted GMRES(m) with right preconditioning. Expects the state's start
 // (rnorm0, threshold, done, iter) set, r = b - A x and b the right-hand side.
-// One host poll per restart cycle; the steps of a cycle after it ended are
-// launched but return at once.
+// The host polls at the end of a restart cycle and where the residual's rate says
+// that the cycle should end; steps launched after its end return at once.
 template <typename XT, int PRE>
 static cfd_status gmres_loop(Launcher& lc, cfd_csr* a, cfd_amg* amg, KrylovBufs<XT>& B, DevState* st, Poller& pl,
                              int64_t restart) {

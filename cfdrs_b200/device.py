@@ -45,8 +45,10 @@ class Context:
         _lib.check(_lib.load().cfd_context_synchronize(self.h))
 
     def set_cluster_solve(self, enable: bool) -> None:
-        """Whole CG / Jacobi-PCG solves of small systems in one thread-block
-        cluster launch (the default) or always the multi-kernel solve."""
+        """Whole CG / Jacobi-PCG and FP64 GMRES solves of small systems in one
+        thread-block cluster or cooperative launch, and GMRES's Arnoldi steps
+        of small systems in one cluster launch (the default), or always the
+        multi-kernel solve."""
         _lib.check(_lib.load().cfd_context_set_cluster_solve(self.h, 1 if enable else 0))
 
     def kernel_stats(self) -> dict:

@@ -79,8 +79,11 @@ cfd_status cfd_context_set_stream(cfd_context* ctx, void* cuda_stream);
 /* FP64 CG and Jacobi-PCG (cfd_solve) of a system whose rows fit the shared
  * memory of one thread-block cluster (up to 16 CTAs; e.g. 16 384 rows of a
  * 5-point operator) run as one launch, the whole recurrence on chip
- * (enable != 0, the default); 0 keeps the multi-kernel solve for every size.
- * Same recurrence and termination; the dot products sum in another order. */
+ * (enable != 0, the default); larger ones whose rows fit the registers and shared
+ * memory of the device run as one cooperative launch, FP64 GMRES (plain, Jacobi or
+ * AMG) of a system that fits a cluster as one launch, and other GMRES
+ * solves of up to 16 384 rows form each Arnoldi step in one cluster launch. 0
+ * keeps the multi-kernel solve for every size. Same recurrence and termination; the dot products sum in another order. */
 cfd_status cfd_context_set_cluster_solve(cfd_context* ctx, int32_t enable);
 cfd_status cfd_context_synchronize(cfd_context* ctx);
 cfd_status cfd_context_destroy(cfd_context* ctx);
@@ -435,6 +438,8 @@ cfd_status cfd_batch_solve(cfd_batch* batch, const cfd_solve_options* opt, const
  *   |d_ii| <= f64::EPSILON), IterativeSolverConfig::new(tolerance): stop at
  *   ||D b - D A x||_2 <= tolerance or after max_iterations; kept when it
  *   converged and the target above holds, else dense LU of A x = b.
+ * An LU runs along the pattern's sparse elimination plan (diagonal pivots, every
+ * multiplier checked) where the pattern has one, else densely.
  * Not restated: the QR least-squares solve the reference tries when a dense LU
  * meets a zero pivot; such a system is reported CFD_LS_PATH_FAILED. A
  * non-finite diagonal of D A (DiagJacobi::new's Err) is CFD_LS_PATH_ERROR.
