@@ -165,10 +165,6 @@ __device__ __forceinline__ int gc_u16(uint32_t a) {
 __device__ __forceinline__ void gc_st(uint32_t a, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
-__device__ __forceinline__ void gc_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 struct GcCta {
   unsigned char* sm;
@@ -352,12 +348,12 @@ __device__ __noinline__ void gc_run(const GcPhase* __restrict__ prog, int phases
         fetch();
       }
     } else {
-      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      cluster_arrive();
       if (more) {
         P = prog[q + 1];
         fetch();
       }
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      cluster_wait();
     }
   }
 }
@@ -405,7 +401,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) k_cluster_gmres(const __grid_co
       }
       gc_stage_diag(A.solo[l], true, C);
     }
-    gc_barrier();
+    cluster_barrier();
     // the tail's matrix: the tail's cycle on this CTA's share of the unit
     // vectors, each column's entries sent to the CTAs that own their rows
     if (A.solo_levels > 0) {
@@ -447,7 +443,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) k_cluster_gmres(const __grid_co
       s = __shfl_sync(0xffffffffu, warp_sum(s), 0);
       if (lane < C.ncta) gc_st(gc_map(C.base + po + 8u * (uint32_t)(k * kGcMaxCtas + C.rank), (uint32_t)lane), s);
     }
-    gc_barrier();
+    cluster_barrier();
     const double* p = C.d((int)po);
     if (tid < nv) {
       double s = 0.0;
@@ -471,7 +467,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) k_cluster_gmres(const __grid_co
       t = __shfl_sync(0xffffffffu, warp_sum(t), 0);
       if (lane < C.ncta) gc_st(gc_map(C.base + po + 8u * (uint32_t)C.rank, (uint32_t)lane), t);
     }
-    gc_barrier();
+    cluster_barrier();
     const double* p = C.d((int)po);
     double t = 0.0;
     for (int c = 0; c < C.ncta; ++c) t += p[c];
@@ -481,7 +477,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) k_cluster_gmres(const __grid_co
   // w = b - A x for the x in global memory (own rows gathered through o_x0).
   auto residual = [&]() {
     for (int i = tid; i < nr; i += kGcThreads) C.d(o_x0)[i] = A.x[r0 + i];
-    gc_barrier();
+    cluster_barrier();
     gc_spmv(A.M, C.base, nr, o_x0, [&](int i, double s) { w[i] = A.b[r0 + i] - s; });
     __syncthreads();
   };
@@ -494,7 +490,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) k_cluster_gmres(const __grid_co
       return A.o_z;
     } else {
       for (int i = tid; i < nr; i += kGcThreads) C.d(o_x0)[i] = PRE == kGcJacobi ? u[i] * A.jinv[r0 + i] : u[i];
-      gc_barrier();
+      cluster_barrier();
       return o_x0;
     }
   };
@@ -504,7 +500,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) k_cluster_gmres(const __grid_co
   int iter, term;
   const int max_iter = A.st->max_iter;
   bool done = false;
-  gc_barrier();  // matrices and diagonals staged, every CTA running
+  cluster_barrier();  // matrices and diagonals staged, every CTA running
   if (!A.resume) {
     residual();
     rn0 = rn = sqrt(norm2(w));
@@ -609,7 +605,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) k_cluster_gmres(const __grid_co
         __syncwarp();
       }
     }
-    gc_barrier();
+    cluster_barrier();
     // x += M^-1 (V y); r = b - A x; the true residual decides (k_gmres_check)
     for (int i = tid; i < nr; i += kGcThreads) {
       const double* vi = V + i;
@@ -621,7 +617,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) k_cluster_gmres(const __grid_co
     __syncthreads();
     const int z = precond(w);
     for (int i = tid; i < nr; i += kGcThreads) A.x[r0 + i] = A.x[r0 + i] + C.d(z)[i];
-    gc_barrier();  // z read before the residual's gather buffer is written
+    cluster_barrier();  // z read before the residual's gather buffer is written
     residual();
     rn = sqrt(norm2(w));
     if (!isfinite(rn)) {
@@ -646,7 +642,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) k_cluster_gmres(const __grid_co
     st->term = term;
     st->done = done ? 1 : 0;
   }
-  gc_barrier();  // no CTA leaves while its shared memory may still be read
+  cluster_barrier();  // no CTA leaves while its shared memory may still be read
 }
 
 size_t gc_round16(size_t b) { return (b + 15) / 16 * 16; }

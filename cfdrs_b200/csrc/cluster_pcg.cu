@@ -103,10 +103,6 @@ __device__ __forceinline__ void cl_ld_if(double& v, uint32_t a, bool on) {
                : "+d"(v)
                : "r"(a), "r"((int)on));
 }
-__device__ __forceinline__ void cl_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 template <int R>
 __global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
@@ -157,7 +153,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
       sp(1)[i] = x[u];
     }
   }
-  cl_barrier();  // every CTA's x staged (in z and the second p buffer)
+  cluster_barrier();  // every CTA's x staged (in z and the second p buffer)
 
   // Up to two rows a thread keep their first kClU entries in registers: read
   // from shared memory every iteration they bound the SpMV (12 of 20 bytes an
@@ -285,7 +281,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
       t = fold(red[up][lane & 15]);
       if ((lane & 15) == 0) part[slot][up] = t;
     }
-    cl_barrier();
+    cluster_barrier();
     if (warp == 0) {
       t = 0.0;
       cl_ld_if(t, cl_map(pbase + (uint32_t)(slot * 2 + up) * 8u, (uint32_t)(lane & 15)), (lane & 15) < ncta);
@@ -303,7 +299,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
   // second p buffer, the old p in the first is zero)
   double arr = 0.0, arz = 0.0;
   row_sums(0, 0.0, q);
-  cl_barrier();  // x gathered by every CTA before z takes its place
+  cluster_barrier();  // x gathered by every CTA before z takes its place
 #pragma unroll
   for (int u = 0; u < R; ++u) {
     const int i = tid + u * kClThreads;
@@ -401,7 +397,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
     st->term = term;
     st->done = 1;
   }
-  cl_barrier();  // no CTA leaves while its shared memory may still be read
+  cluster_barrier();  // no CTA leaves while its shared memory may still be read
 }
 
 template <int R>

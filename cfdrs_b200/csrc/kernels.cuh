@@ -78,6 +78,23 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// Cluster barrier (release and acquire) of all threads of the cluster. The aligned
+// forms want the whole warp at the instruction, so each is behind a __syncwarp: the
+// code before a barrier may have taken its lanes apart. Control flow around them is
+// uniform in the warp. (Measured against the aligned forms alone: the same time.)
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  cluster_arrive();
+  cluster_wait();
+}
+
 // Sum over the CTA; the result is valid in thread 0.
 template <typename T>
 __device__ __forceinline__ T block_sum(T v) {

@@ -476,18 +476,6 @@ constexpr int kOrthWidth = 256;   // largest restart width (gmres_width)
 constexpr int kOrthLoads = 8;     // loads of a lane in flight
 inline bool orth_fits(int64_t n, int nv) { return n <= kOrthCtas * kOrthRows && nv <= kOrthWidth && n * nv <= 1 << 20; }
 
-__device__ __forceinline__ void cluster_arrive() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-  __syncwarp();
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_barrier() {
-  cluster_arrive();
-  cluster_wait();
-}
 __device__ __forceinline__ double orth_pull(const double* p, uint32_t rank) {
   uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
   double v;
