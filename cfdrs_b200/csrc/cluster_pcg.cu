@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
 template <int R>
 cfd_status cl_launch(cfd_context* ctx, const ClusterArgs& args, int ncta, size_t bytes, bool* launched) {
   auto kern = k_cluster_pcg<R>;
-  CFD_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  CFD_TRY(allow_dynamic_smem(kern, ctx->device));
   if (ncta > 8) CFD_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfgl = {};
   cfgl.gridDim = dim3(ncta);

@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kGpThreads, 1) k_grid_pcg(GridArgs A) {
 template <int R>
 cfd_status gp_launch(cfd_context* ctx, GridArgs& A, int grid, size_t bytes, bool probe, bool* fits) {
   auto kern = k_grid_pcg<R>;
-  CFD_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  CFD_TRY(allow_dynamic_smem(kern, ctx->device));
   if (probe) {
     int occ = 0;
     CFD_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kGpThreads, bytes));

@@ -356,6 +356,21 @@ struct cfd_csr {
 };
 
 namespace cfd {
+// Lets a kernel take all the dynamic shared memory the device has beside its static
+// arrays. A launch states its own size; the limit belongs to the function on the
+// device and the lock of a solve to its context, so a limit set to one call's size
+// could be lowered by another context's call before this one's launch.
+template <class Kernel>
+cfd_status allow_dynamic_smem(Kernel kern, int device) {
+  cudaFuncAttributes fa;
+  int optin = 0;
+  CFD_TRY_CUDA(cudaFuncGetAttributes(&fa, kern));
+  CFD_TRY_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  CFD_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    optin - (int)fa.sharedSizeBytes));
+  return CFD_OK;
+}
+
 cfd_status ensure_partials(cfd_context* ctx, int blocks);
 // Reads the device error flag; a set flag (a bounded wait ran out) is reported
 // as CFD_ERR_TIMEOUT and the flag and reduction ticket are reset.

@@ -460,7 +460,7 @@ cfd_status dense_inverse_device(cfd_context* ctx, int64_t n64, const int* rp, co
   }
   const int ldw = (n + 2) & ~1;
   const size_t smem = (size_t)2 * ldw * sizeof(double) + (size_t)2 * n * sizeof(int);
-  CFD_TRY_CUDA(cudaFuncSetAttribute(k_gj_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CFD_TRY(allow_dynamic_smem(k_gj_coop, ctx->device));
   int occ = 0;
   CFD_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_gj_coop, kGjThreads, smem));
   if (occ < 1) {
