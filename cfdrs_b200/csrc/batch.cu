@@ -349,8 +349,12 @@ __host__ __device__ constexpr size_t batch_reg_p_off(int nmax, int zmax) {
   return batch_reg_rp_off<T>(zmax) + round16((size_t)(nmax + 1) * 2);
 }
 template <typename T>
+__host__ __device__ constexpr size_t batch_reg_jinv_off(int nmax, int zmax) {  // behind p and a slot that stays zero
+  return batch_reg_p_off<T>(nmax, zmax) + round16((size_t)(nmax + 1) * sizeof(T));
+}
+template <typename T>
 __host__ __device__ constexpr size_t batch_reg_smem(int nmax, int zmax) {
-  return batch_reg_p_off<T>(nmax, zmax) + 2 * round16((size_t)nmax * sizeof(T));
+  return batch_reg_jinv_off<T>(nmax, zmax) + round16((size_t)nmax * sizeof(T));
 }
 
 // group_sum of two values at once, each in group_sum's order (an exclusive-or
@@ -391,7 +395,7 @@ __global__ void __launch_bounds__(kRegThreads) k_batch_pcg_reg(BatchSys S, Batch
   unsigned short* sc = reinterpret_cast<unsigned short*>(sm + batch_reg_col_off<T>(zmax));
   unsigned short* srp = reinterpret_cast<unsigned short*>(sm + batch_reg_rp_off<T>(zmax));
   T* vp = reinterpret_cast<T*>(sm + batch_reg_p_off<T>(nmax, zmax));
-  T* vj = reinterpret_cast<T*>(sm + batch_reg_p_off<T>(nmax, zmax) + round16((size_t)nmax * sizeof(T)));
+  T* vj = reinterpret_cast<T*>(sm + batch_reg_jinv_off<T>(nmax, zmax));
   __shared__ double reds[kMaxGroups][2][2][32];
   __shared__ int s_ks[kMaxGroups];
   double(*red)[2][32] = reds[G.g];
@@ -418,10 +422,10 @@ __global__ void __launch_bounds__(kRegThreads) k_batch_pcg_reg(BatchSys S, Batch
       sv[e] = REFINE ? (T)S.v32[k0 + e] : (T)S.v64[k0 + e];
       sc[e] = (unsigned short)S.col[k0 + e];
     }
-    if (tid == 0) {  // the zero entry: row 0's direction times 0
+    if (tid == 0) {  // the zero entry: a slot that stays zero, times 0
       sv[zmax] = T(0);
-      sc[zmax] = 0;
-      vp[0] = T(0);
+      sc[zmax] = (unsigned short)nmax;
+      vp[nmax] = T(0);
     }
     gsync();
 #pragma unroll

@@ -477,8 +477,12 @@ __host__ __device__ constexpr size_t ls_reg_vec_off(int nmax, int zmax) {
   return ls_reg_rp_off<T>(zmax) + ls_round16((size_t)(nmax + 1) * 2);
 }
 template <typename T>
+__host__ __device__ constexpr size_t ls_reg_inv_off(int nmax, int zmax) {  // behind w and a slot that stays zero
+  return ls_reg_vec_off<T>(nmax, zmax) + ls_round16((size_t)(nmax + 1) * sizeof(T));
+}
+template <typename T>
 __host__ __device__ constexpr size_t ls_reg_smem(int nmax, int zmax) {
-  return ls_reg_vec_off<T>(nmax, zmax) + 2 * ls_round16((size_t)nmax * sizeof(T));
+  return ls_reg_inv_off<T>(nmax, zmax) + ls_round16((size_t)nmax * sizeof(T));
 }
 
 // ls_cta_sum2 in its order (an exclusive-or butterfly adds the same pairs as the
@@ -521,7 +525,7 @@ __global__ void __launch_bounds__(kLsRegThreads, 2) k_ls_krylov_reg(LsArgs A, co
   unsigned short* sc = reinterpret_cast<unsigned short*>(sm + ls_reg_col_off<T>(zmax));
   unsigned short* srp = reinterpret_cast<unsigned short*>(sm + ls_reg_rp_off<T>(zmax));
   T* vw = reinterpret_cast<T*>(sm + ls_reg_vec_off<T>(nmax, zmax));
-  T* vinv = reinterpret_cast<T*>(sm + ls_reg_vec_off<T>(nmax, zmax) + ls_round16((size_t)nmax * sizeof(T)));
+  T* vinv = reinterpret_cast<T*>(sm + ls_reg_inv_off<T>(nmax, zmax));
   constexpr int U = 4;               // entries of a row read together
   constexpr int W = R >= 2 ? 2 : 1;  // rows side by side
   T vx[R], vr[R], vrh[R], vp[R], vv[R], vt[R];
@@ -548,10 +552,10 @@ __global__ void __launch_bounds__(kLsRegThreads, 2) k_ls_krylov_reg(LsArgs A, co
     const int k0 = A.rp[r0], nnz = A.rp[r0 + n] - k0;
     for (int i = tid; i <= n; i += nt) srp[i] = (unsigned short)(A.rp[r0 + i] - k0);
     for (int e = tid; e < nnz; e += nt) sc[e] = (unsigned short)A.col[k0 + e];
-    if (tid == 0) {  // the zero entry: entry 0 of the gathered vector times 0
+    if (tid == 0) {  // the zero entry: a slot that stays zero, times 0
       sv[zmax] = T(0);
-      sc[zmax] = 0;
-      vw[0] = T(0);
+      sc[zmax] = (unsigned short)nmax;
+      vw[nmax] = T(0);
     }
 #pragma unroll
     for (int u = 0; u < R; ++u) vx[u] = vr[u] = vrh[u] = vp[u] = vv[u] = vt[u] = T(0);

@@ -191,7 +191,7 @@ __device__ void gc_stage(const GcMat& A, const GcCta& C) {
     v[e] = A.val[k0 + e];
   }
   if (threadIdx.x == 0) {
-    cl[A.zero] = (uint16_t)(C.rank << kGcIdxBits);  // this CTA's slice of any vector: finite from the start
+    cl[A.zero] = (uint16_t)((C.rank << kGcIdxBits) | A.rpc_c);  // the slot behind this CTA's slice: stays zero
     v[A.zero] = 0.0;
   }
 }
@@ -206,7 +206,8 @@ __device__ void gc_stage_diag(const GcLevel& L, bool solo, const GcCta& C) {
 
 // A row's entries ka, ka + step, ... below ke of a matrix, U at a time: values
 // and the gathered entries' cluster addresses. Slots past the end take the
-// matrix's zero entry, so the loads carry no branches and overlap.
+// matrix's zero entry, so the loads carry no branches and overlap; it names a slot
+// of the vector that stays zero, so no vector entry reaches a row without its column.
 constexpr int kGcU = 5;  // a five-point row in one batch
 struct GcBatch {
   double v[kGcU];
@@ -700,7 +701,7 @@ size_t gc_layout(GcArgs& A, const HostCsr& op, const cfd_amg* amg, int pre, int 
     const int t = A.levels - 1;
     for (int l = 0; l < A.levels; ++l) {
       GcLevel& L = A.lev[l];
-      const size_t vb = (size_t)L.rpc * 8;
+      const size_t vb = (size_t)(L.rpc + 1) * 8;  // and a zero behind the slice
       L.o_xa = take(vb);
       L.o_b = l == 0 ? A.o_w : take(vb);
       L.o_d = take(vb);
@@ -718,7 +719,7 @@ size_t gc_layout(GcArgs& A, const HostCsr& op, const cfd_amg* amg, int pre, int 
       GcLevel& L = A.solo[l];
       const HostLevel& H = amg->host[t + l];
       L.n = L.rpc = (int)H.A.nrows;
-      const size_t vb = (size_t)L.n * 8;
+      const size_t vb = (size_t)(L.n + 1) * 8;
       mat(L.A, H.A, L.n, L.n, true, nullptr);
       if (l + 1 < A.solo_levels) {
         const int nc = (int)amg->host[t + l + 1].A.nrows;
@@ -735,7 +736,7 @@ size_t gc_layout(GcArgs& A, const HostCsr& op, const cfd_amg* amg, int pre, int 
     A.o_prog = take((size_t)(A.phases + A.solo_phases) * sizeof(GcPhase));
     A.o_stage = take((size_t)A.lev[t].n * 8);
   } else {
-    A.lev[0].o_xa = take((size_t)A.rpc * 8);
+    A.lev[0].o_xa = take((size_t)(A.rpc + 1) * 8);
   }
   const size_t mv = (size_t)(A.m + 1) * 8;
   A.o_part = take(2 * mv * kGcMaxCtas);

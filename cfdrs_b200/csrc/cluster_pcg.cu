@@ -19,7 +19,8 @@
 //    throughput is low even for a CTA's own memory (SpMV phase 1600 -> 1190
 //    cycles at 128^2).
 //  - A row's five entries are read without branches (slots past its end take a
-//    zero entry), so all of its gathers are in flight together.
+//    zero entry, value 0 times a vector slot that stays 0, so that no vector entry
+//    reaches a row without its column), so all of its gathers are in flight together.
 //  - Behind a reduction's barrier one warp fetches the CTAs' partials (one
 //    remote load) and hands the totals to the others; pushing them to every CTA
 //    before the barrier made the barrier wait for the stores (3.65 against 3.08
@@ -85,7 +86,7 @@ __host__ __device__ inline ClusterLayout cluster_layout(int rpc, int nnz_cap) {
   L.rpl = L.ent + cl_round16((size_t)(nnz_cap + 1) * 4);
   L.z = L.rpl + cl_round16((size_t)(rpc + 1) * 4);
   L.p = L.z + cl_round16((size_t)rpc * 8);
-  L.bytes = L.p + 2 * cl_round16((size_t)rpc * 8);  // two buffers
+  L.bytes = L.p + 2 * cl_round16((size_t)(rpc + 1) * 8);  // two buffers, each with a slot that stays zero
   return L;
 }
 
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
   int* sent = reinterpret_cast<int*>(sm + L.ent);  // owner << 16 | local index
   int* srp = reinterpret_cast<int*>(sm + L.rpl);
   double* sz = reinterpret_cast<double*>(sm + L.z);
-  const uint32_t psz = (uint32_t)cl_round16((size_t)A.rpc * 8);  // bytes of a p buffer
+  const uint32_t psz = (uint32_t)cl_round16((size_t)(A.rpc + 1) * 8);  // bytes of a p buffer
   auto sp = [&](int buf) { return reinterpret_cast<double*>(sm + L.p + (buf ? psz : 0u)); };
   __shared__ double part[2][2];  // [slot][value]: this CTA's partial sums
   __shared__ double bcast[2];
@@ -135,9 +136,10 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
     sent[e] = (owner << 16) | (c - owner * A.rpc);
     sval[e] = A.val[k0 + e];
   }
-  if (tid == 0) {  // the zero entry: this CTA's first vector entry times 0
-    sent[A.nnz_cap] = rank << 16;
+  if (tid == 0) {  // the zero entry
+    sent[A.nnz_cap] = (rank << 16) | A.rpc;
     sval[A.nnz_cap] = 0.0;
+    sp(0)[A.rpc] = sp(1)[A.rpc] = 0.0;
   }
   double x[R], r[R], p[R], q[R], jv[R];
 #pragma unroll

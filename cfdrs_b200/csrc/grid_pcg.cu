@@ -76,7 +76,7 @@ __host__ __device__ inline GridLayout grid_layout(int rpc, int nnz_cap, int far_
   L.rpl = L.ent + gp_round16((size_t)(nnz_cap + 1) * 4);
   L.far = L.rpl + gp_round16((size_t)(rpc + 1) * 4);
   L.p = L.far + gp_round16((size_t)far_cap * 4);
-  L.bytes = L.p + gp_round16((size_t)(rpc + far_cap) * 8);
+  L.bytes = L.p + gp_round16((size_t)(rpc + far_cap + 1) * 8);  // and a slot that stays zero
   return L;
 }
 
@@ -133,10 +133,10 @@ __global__ void __launch_bounds__(kGpThreads, 1) k_grid_pcg(GridArgs A) {
     sent[e] = slot;
     sval[e] = A.val[k0 + e];
   }
-  if (tid == 0) {  // the zero entry: this CTA's first direction entry times 0
-    sent[A.nnz_cap] = 0;
+  if (tid == 0) {  // the zero entry: a slot that stays zero, times 0
+    sent[A.nnz_cap] = A.rpc + A.far_cap;
     sval[A.nnz_cap] = 0.0;
-    sp[0] = 0.0;
+    sp[A.rpc + A.far_cap] = 0.0;
   }
   const int iter0 = A.first ? 0 : A.st->iter;
   double x[R], r[R], p[R], q[R], jv[R];
