@@ -148,6 +148,8 @@ cfd_status devmat_upload(DevMat& m, const HostCsr& h, bool want32, cudaStream_t 
   }
   std::vector<int> rp32(h.nrows + 1);
   for (int64_t i = 0; i <= h.nrows; ++i) rp32[i] = (int)h.rp[i];
+  m.max_row = 0;
+  for (int64_t i = 0; i < h.nrows; ++i) m.max_row = std::max(m.max_row, rp32[i + 1] - rp32[i]);
   m.tpr = threads_per_row(m.nnz, m.nrows);
   std::vector<int> blk = row_partition(h.rp.data(), h.nrows, m.tpr);
   m.nblk = (int)blk.size() - 1;

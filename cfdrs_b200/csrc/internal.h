@@ -169,6 +169,7 @@ struct DevMat {
   mutable int8_t path[2] = {-1, -1};
   int nblk = 0;
   int tpr = 1;         // threads cooperating on one row (power of two, <= 32)
+  int max_row = 0;     // entries of the longest row
   // Sliced layout (FP32 SpMV only; HostSliced): slice offsets, codes,
   // dictionaries, the CSR entry of every slot and the slot-major FP32 values,
   // gathered from v32 before the first sliced SpMV after v32 changed.

@@ -843,12 +843,18 @@ struct Launcher {
   // sides measured by moving the limit: 512^2 adjoint 8.03 ms without the kernel,
   // 7.23 / 7.10 / 7.00 / 6.95 ms up to 0.1 / 0.3 / 0.8 / 3 M FP32 entries; 96^3 FP64
   // 3.28 ms without, 3.24 ms to 0.8 M, 3.27 to 3 M, 3.33 to 12 M; 192^3 FP32 14.89 ms
-  // without, 14.70 to 3 M, 15.07 to 12 M.
+  // without, 14.70 to 3 M, 15.07 to 12 M. And no row of more than 48 entries a
+  // thread: a row group reads its row from global memory batch after batch, where the
+  // pipelines have it staged (a row past a block's capacity by the whole CTA). CG of
+  // 20 000 rows of 5 with one long row, us an iteration with the kernel / without:
+  // FP64 16.2 / 17.5 at 35 entries, 20.9 / 21.5 at 67, 49 / 42 at 256; FP32 38.5 /
+  // 39.5, 47 / 44, 105 / 66; two and four threads a row: ahead at 40 entries a thread,
+  // even at 68. A row of 50 000 took 6605 us against 39.
   template <typename VT>
   static bool direct_fits(const DevMat& m, int p, int nred) {
     const int64_t grid = (m.nrows * (int64_t)m.tpr + kThreads - 1) / kThreads;
     return m.path[p] == CFD_PATH_AUTO && m.nnz * (int64_t)(sizeof(VT) + 4) <= (int64_t)16 << 20 &&
-           (nred == 0 || grid <= kVecGrid);
+           m.max_row <= 48 * m.tpr && (nred == 0 || grid <= kVecGrid);
   }
   static constexpr int kPathTimed = -2, kPathSplit = 0, kPathRecord = 1, kPathXs = 2, kPathSliced = 3,
                        kPathDiag = 4;
