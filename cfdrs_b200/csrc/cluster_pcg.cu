@@ -61,6 +61,7 @@ constexpr int kClWarps = kClThreads / 32;
 constexpr int kClMaxCtas = 16;
 constexpr int kClMaxRows = 8;  // rows per thread
 constexpr int kClU = 5;        // entries of a row read together (a five-point row)
+constexpr int kClMaxFar = 1500;  // scattered entries of other CTAs (cluster_pcg_solve)
 
 struct ClusterArgs {
   const int* __restrict__ rp;  // global CSR (int32)
@@ -263,8 +264,9 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_pcg(ClusterArgs A) {
       for (int g = 0; g < G; ++g) out[u0 + g] = s[g];
     }
   };
-  // CTA partials pushed to every CTA, one barrier, then summed in rank order:
-  // every CTA gets the same bits. Two slots in turn: a CTA pushes into a slot
+  // Sums over the cluster: each CTA leaves its partials in a slot of its own, and
+  // behind one barrier a warp of every CTA fetches all of them and folds them in the
+  // same butterfly, so all hold the same bits. Two slots in turn: a CTA writes one
   // again only after a barrier that the others pass behind their reads of it.
   int slot = 0;
   auto totals = [&](double a, double b2, double& ta, double& tb) {
@@ -432,12 +434,39 @@ cfd_status cl_launch(cfd_context* ctx, const ClusterArgs& args, int ncta, size_t
 
 }  // namespace
 
+int64_t scattered_far(const HostCsr& h, int rpc) {
+  int64_t cap = 0;
+  for (int64_t r = 0; r < h.nrows; r += rpc) {
+    const int64_t e = std::min<int64_t>(r + rpc, h.nrows);
+    int64_t far = 0;
+    for (int64_t i = r; i < e; ++i) {
+      const int64_t up = i > r ? h.rp[i] - h.rp[i - 1] : 0;
+      for (int64_t k = h.rp[i]; k < h.rp[i + 1]; ++k)
+        if (h.ci[k] < r || h.ci[k] >= e)
+          far += k - h.rp[i] >= up || h.ci[k - up] + 1 != h.ci[k];
+    }
+    cap = std::max(cap, far);
+  }
+  return cap;
+}
+
 // The cluster solve applies when the system's rows, split over at most 16
-// CTAs, fit their shared memory and registers; *ok = false otherwise (nothing
-// launched).
-cfd_status cluster_pcg_solve(cfd_context* ctx, const HostCsr& h, const DevMat& m, const double* jinv, const double* b,
-                             double* x, DevState* st, bool* ok) {
+// CTAs, fit their shared memory and registers, and no CTA gathers more than
+// kClMaxFar scattered entries from others; *ok = false otherwise (nothing
+// launched). What bounds it beyond that is the throughput of remote loads, two an
+// entry (about 4.5 ns each where the columns are scattered; a stencil's
+// neighbouring rows share theirs), where the grid form stays at 6 to 8 us an
+// iteration. Us an iteration in a cluster / on the grid / multi-kernel:
+//    1031 scattered entries (1000 rows)   5.7 / 6.7 / 12.9
+//    1458 ( 300 rows)                     5.5 / 7.2 / 16.3
+//    1563 (2000 rows)                     7.6 / 6.7 / 13.3
+//    4794 (8000 rows)                    27.3 / 7.8 / 15.4
+//   27-point 16^3 (4232, most of them in runs)  5.8 / 7.3 / 21.3
+cfd_status cluster_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, const double* b, double* x, DevState* st,
+                             bool* ok) {
   *ok = false;
+  const HostCsr& h = a->host;
+  const DevMat& m = a->dev;
   const int64_t n = m.nrows;
   if (n <= 0 || n > (int64_t)kClMaxCtas * kClThreads * kClMaxRows || m.nrows != m.ncols) return CFD_OK;
   int max_smem = 0;
@@ -453,6 +482,11 @@ cfd_status cluster_pcg_solve(cfd_context* ctx, const HostCsr& h, const DevMat& m
     for (int64_t r = 0; r < n; r += rpc) nnz_cap = std::max(nnz_cap, h.rp[std::min<int64_t>(r + rpc, n)] - h.rp[r]);
     const ClusterLayout L = cluster_layout(rpc, (int)std::min<int64_t>(nnz_cap, 1 << 24));
     if (L.bytes > budget) continue;
+    if (a->cluster_far_rows != rpc) {  // follows from the pattern, which a matrix keeps for life
+      a->cluster_far = scattered_far(h, rpc);
+      a->cluster_far_rows = rpc;
+    }
+    if (a->cluster_far > kClMaxFar) return CFD_OK;
     ClusterArgs args{m.rp, m.col, m.v64, jinv, b, x, st, (int)n, rpc, (int)nnz_cap};
     const int rows = (rpc + kClThreads - 1) / kClThreads;
     if (rows <= 1)

@@ -354,6 +354,9 @@ struct cfd_csr {
   // Boundary entries of the fullest row block of the grid CG (grid_pcg.cu), -1
   // before its first use; a function of the pattern and the GPU's SM count.
   int64_t grid_far = -1;
+  // scattered_far of the cluster CG's row blocks, and their rows (0: not counted yet).
+  int64_t cluster_far = 0;
+  int cluster_far_rows = 0;
 };
 
 namespace cfd {
@@ -384,8 +387,12 @@ cfd_status csr_sync_host(cfd_csr* a);
 cfd_status pattern_outer_launch(cfd_csr* a, const double* lambda, const double* x, double scale, double* g);
 // Whole CG / Jacobi-PCG solve in one thread-block cluster (cluster_pcg.cu):
 // *ok = false (nothing launched) when the system does not fit.
-cfd_status cluster_pcg_solve(cfd_context* ctx, const HostCsr& h, const DevMat& m, const double* jinv, const double* b,
-                             double* x, DevState* st, bool* ok);
+cfd_status cluster_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, const double* b, double* x, DevState* st,
+                             bool* ok);
+// Scattered entries outside the block of the fullest of the row blocks of rpc rows:
+// an entry that continues the entry at its place in the row above (column one
+// further, as in a stencil) is not scattered.
+int64_t scattered_far(const HostCsr& h, int rpc);
 // CG / Jacobi-PCG on one cooperative grid (grid_pcg.cu), for systems beyond a
 // cluster: *ok = false (nothing launched) when the system does not fit.
 cfd_status grid_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, const double* b, double* x, DevState* st,

@@ -1541,8 +1541,7 @@ cfd_status solve_fp64(cfd_csr* a, const cfd_solve_options& opt, cfd_amg* amg, co
   const bool plain_pre = opt.precond == CFD_PRECOND_NONE || opt.precond == CFD_PRECOND_JACOBI;
   bool whole = false;
   if (ctx->cluster_solve && opt.solver == CFD_SOLVER_CG && plain_pre)
-    CFD_TRY(cluster_pcg_solve(ctx, a->host, a->dev, opt.precond == CFD_PRECOND_JACOBI ? a->jinv64 : nullptr, B.b, B.x,
-                              st, &whole));
+    CFD_TRY(cluster_pcg_solve(ctx, a, opt.precond == CFD_PRECOND_JACOBI ? a->jinv64 : nullptr, B.b, B.x, st, &whole));
   if (ctx->cluster_solve && opt.solver == CFD_SOLVER_CG && plain_pre && !whole)
     CFD_TRY(grid_pcg_solve(ctx, a, opt.precond == CFD_PRECOND_JACOBI ? a->jinv64 : nullptr, B.b, B.x, st, hs, &whole));
   if (ctx->cluster_solve && opt.solver == CFD_SOLVER_GMRES && (plain_pre || opt.precond == CFD_PRECOND_AMG))
