@@ -824,8 +824,10 @@ void gc_programs(GcArgs& A, const cfd_amg_config& c, std::vector<GcPhase>& prog)
 template <int PRE>
 cfd_status gc_launch(cfd_context* ctx, const GcArgs& A, int ncta, size_t smem, bool probe, bool* fits) {
   auto kern = k_cluster_gmres<PRE>;
-  CFD_TRY(allow_dynamic_smem(kern, ctx->device));
-  if (ncta > 8) CFD_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  if (probe) {  // once a solve, before its launches
+    CFD_TRY(allow_dynamic_smem(kern, ctx->device));
+    if (ncta > 8) CFD_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ncta);
   cfg.blockDim = dim3(kGcThreads);

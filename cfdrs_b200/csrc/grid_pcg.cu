@@ -404,8 +404,8 @@ __global__ void __launch_bounds__(kGpThreads, 1) k_grid_pcg(GridArgs A) {
 template <int R>
 cfd_status gp_launch(cfd_context* ctx, GridArgs& A, int grid, size_t bytes, bool probe, bool* fits) {
   auto kern = k_grid_pcg<R>;
-  CFD_TRY(allow_dynamic_smem(kern, ctx->device));
-  if (probe) {
+  if (probe) {  // once a solve, before its launches
+    CFD_TRY(allow_dynamic_smem(kern, ctx->device));
     int occ = 0;
     CFD_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kGpThreads, bytes));
     *fits = occ >= 1;
