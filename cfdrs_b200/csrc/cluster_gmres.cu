@@ -66,6 +66,7 @@ constexpr int kGcIdxBits = 12;          // local index bits of a packed column
 constexpr int kGcMaxDense = 512;        // rows of a dense coarsest solve at most
 constexpr int kGcStepsPerLaunch = 4096;
 constexpr int kGcMaxPhases = 128;
+constexpr int kGcMaxFar = 14000;        // scattered entries of other CTAs (cluster_gmres_solve)
 
 enum { kGcNone = 0, kGcJacobi = 1, kGcAmg = 2 };
 
@@ -866,7 +867,15 @@ cfd_status gc_launch_pre(cfd_context* ctx, int pre, const GcArgs& A, int ncta, s
 // split over at most 16 CTAs fits their shared memory; *ok = false otherwise
 // (nothing launched). x holds the initial guess and takes the solution; the
 // state takes the outcome. m: the restart width (a power of two).
-cfd_status cluster_gmres_solve(cfd_context* ctx, const cfd_csr* a, cfd_amg* amg, int precond, int m, const double* b,
+// Without a V-cycle a step is one SpMV, bound by its remote gathers where the columns
+// are scattered over the CTAs: such a system goes to the separate kernels beyond
+// kGcMaxFar entries of other CTAs in a block. A GMRES(8) of 16 steps, here / separate
+// kernels, ms: 0.82 / 0.92 at 12300 entries, 0.84 / 0.86 and 0.88 / 0.90 at 13800 and
+// 14200, 0.98 / 0.91 at 14800, 1.14 / 0.92 at 17200. With the V-cycle, some fifty
+// launches a step, the cluster was ahead wherever the hierarchy fits (1.13x at least).
+// What bounds the size otherwise is capacity: five-point systems of 48400 rows, the
+// largest that fit, 0.46 / 0.86 ms, tridiagonal ones of 65000 0.58 / 0.85.
+cfd_status cluster_gmres_solve(cfd_context* ctx, cfd_csr* a, cfd_amg* amg, int precond, int m, const double* b,
                                double* x, DevState* st, DevState* host_st, bool* ok) {
   *ok = false;
   const int64_t n = a->dev.nrows;
@@ -909,6 +918,7 @@ cfd_status cluster_gmres_solve(cfd_context* ctx, const cfd_csr* a, cfd_amg* amg,
     if (fits) break;
   }
   if (ncta > kGcMaxCtas) return CFD_OK;
+  if (pre != kGcAmg && cluster_scattered(a, 1, A.rpc) > kGcMaxFar) return CFD_OK;
   const size_t basis = gc_round16((size_t)(m + 1) * A.rpc * 8);
   A.o_v = -1;
   if (smem + basis <= budget) {

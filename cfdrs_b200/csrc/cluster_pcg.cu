@@ -482,11 +482,7 @@ cfd_status cluster_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, c
     for (int64_t r = 0; r < n; r += rpc) nnz_cap = std::max(nnz_cap, h.rp[std::min<int64_t>(r + rpc, n)] - h.rp[r]);
     const ClusterLayout L = cluster_layout(rpc, (int)std::min<int64_t>(nnz_cap, 1 << 24));
     if (L.bytes > budget) continue;
-    if (a->cluster_far_rows != rpc) {  // follows from the pattern, which a matrix keeps for life
-      a->cluster_far = scattered_far(h, rpc);
-      a->cluster_far_rows = rpc;
-    }
-    if (a->cluster_far > kClMaxFar) return CFD_OK;
+    if (cluster_scattered(a, 0, rpc) > kClMaxFar) return CFD_OK;
     ClusterArgs args{m.rp, m.col, m.v64, jinv, b, x, st, (int)n, rpc, (int)nnz_cap};
     const int rows = (rpc + kClThreads - 1) / kClThreads;
     if (rows <= 1)

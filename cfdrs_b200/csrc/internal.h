@@ -354,9 +354,10 @@ struct cfd_csr {
   // Boundary entries of the fullest row block of the grid CG (grid_pcg.cu), -1
   // before its first use; a function of the pattern and the GPU's SM count.
   int64_t grid_far = -1;
-  // scattered_far of the cluster CG's row blocks, and their rows (0: not counted yet).
-  int64_t cluster_far = 0;
-  int cluster_far_rows = 0;
+  // scattered_far of the row blocks of the cluster CG [0] and GMRES [1], and the
+  // blocks' rows (0: not counted yet).
+  int64_t cluster_far[2] = {};
+  int cluster_far_rows[2] = {};
 };
 
 namespace cfd {
@@ -393,12 +394,19 @@ cfd_status cluster_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, c
 // an entry that continues the entry at its place in the row above (column one
 // further, as in a stencil) is not scattered.
 int64_t scattered_far(const HostCsr& h, int rpc);
+inline int64_t cluster_scattered(cfd_csr* a, int form, int rpc) {
+  if (a->cluster_far_rows[form] != rpc) {  // follows from the pattern, which a matrix keeps for life
+    a->cluster_far[form] = scattered_far(a->host, rpc);
+    a->cluster_far_rows[form] = rpc;
+  }
+  return a->cluster_far[form];
+}
 // CG / Jacobi-PCG on one cooperative grid (grid_pcg.cu), for systems beyond a
 // cluster: *ok = false (nothing launched) when the system does not fit.
 cfd_status grid_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, const double* b, double* x, DevState* st,
                           DevState* host_st, bool* ok);
 // Whole GMRES(m) solve (no preconditioner, Jacobi or AMG) in one thread-block
 // cluster (cluster_gmres.cu): *ok = false (nothing launched) when it does not fit.
-cfd_status cluster_gmres_solve(cfd_context* ctx, const cfd_csr* a, cfd_amg* amg, int precond, int m, const double* b,
+cfd_status cluster_gmres_solve(cfd_context* ctx, cfd_csr* a, cfd_amg* amg, int precond, int m, const double* b,
                                double* x, DevState* st, DevState* host_st, bool* ok);
 }  // namespace cfd
