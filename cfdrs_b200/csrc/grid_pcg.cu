@@ -8,9 +8,10 @@
 // SpMV with its reduction 5.3 us, direction 2.4 us at 123 300 rows) on data that
 // sits in L2. Here an iteration is bound by two grid-wide reductions and one
 // exchange of boundary entries, each a store to L2 and the others' polls of it.
-// No fence is on that path: a double travels as two 8-byte words of 32 data and
-// 32 flag bits (the number of the reduction or iteration), so a reader that sees
-// the flag has the data. (With fences around flags and sums read apart the same
+// No fence is on that path: a double travels as NCCL's LL protocol sends data, in
+// two 8-byte words of 32 data and 32 flag bits (the number of the reduction or
+// iteration), each stored and loaded as one 64-bit access, so a reader that sees
+// a word's flag has its data. (With fences around flags and sums read apart the same
 // kernel took 15 us an iteration, more than the three launches' 13.) Measured,
 // five-point Jacobi-CG to 1e-10, before (multi-kernel) and now: 256 x 256 10.6
 // -> 5.4 ms, 411 x 300 18.6 -> 8.8 ms, 600 x 620 46.4 -> 20.1 ms. Half the CTAs
@@ -58,8 +59,8 @@ struct GridArgs {
   double* x;
   double* r;    // residual and direction between launches
   double* p;
-  uint4* z;     // published D^-1 r of all rows
-  uint4* sums;  // published partial sums: two buffers of two per CTA
+  ulonglong2* z;     // published D^-1 r of all rows
+  ulonglong2* sums;  // published partial sums: two buffers of two per CTA
   DevState* st;
   int* err;
   int n, rpc, nnz_cap, far_cap, first;
@@ -80,22 +81,23 @@ __host__ __device__ inline GridLayout grid_layout(int rpc, int nnz_cap, int far_
   return L;
 }
 
-// A double as two 8-byte words, each 32 bits of it and the flag.
-__device__ __forceinline__ void gp_publish(uint4* to, double v, unsigned flag) {
-  const unsigned lo = (unsigned)__double2loint(v), hi = (unsigned)__double2hiint(v);
-  asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(to), "r"(lo), "r"(flag), "r"(hi) : "memory");
-}
-__device__ __forceinline__ bool gp_read(const uint4* from, unsigned flag, double& v) {
-  unsigned lo, f0, hi, f1;
-  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(lo), "=r"(f0), "=r"(hi), "=r"(f1)
-               : "l"(from)
+// A double as two 8-byte words, each 32 bits of it (low) and the flag (high). The
+// elements of the vector access are 64 bits wide: PTX makes no promise for a word
+// made of two 32-bit elements.
+__device__ __forceinline__ void gp_publish(ulonglong2* to, double v, unsigned flag) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(v), f = (unsigned long long)flag << 32;
+  asm volatile("st.volatile.global.v2.b64 [%0], {%1, %2};" ::"l"(to), "l"((bits & 0xffffffffull) | f),
+               "l"((bits >> 32) | f)
                : "memory");
-  v = __hiloint2double((int)hi, (int)lo);
-  return f0 == flag && f1 == flag;
+}
+__device__ __forceinline__ bool gp_read(const ulonglong2* from, unsigned flag, double& v) {
+  unsigned long long a, b;
+  asm volatile("ld.volatile.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(from) : "memory");
+  v = __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
+  return (unsigned)(a >> 32) == flag && (unsigned)(b >> 32) == flag;
 }
 // Polls until the flag is there; false when the wait runs out.
-__device__ __forceinline__ bool gp_wait(const uint4* from, unsigned flag, double& v) {
+__device__ __forceinline__ bool gp_wait(const ulonglong2* from, unsigned flag, double& v) {
   for (unsigned tries = 0; tries < kGpSpin; ++tries)
     if (gp_read(from, flag, v)) return true;
   return false;
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(kGpThreads, 1) k_grid_pcg(GridArgs A) {
     return fold((up ? b2 : a) + got);
   };
   auto totals = [&](unsigned epoch, bool two, double a, double b2, double& ta, double& tb) -> bool {
-    uint4* sums = A.sums + (size_t)(epoch & 1u) * 2 * kGpMaxGrid;
+    ulonglong2* sums = A.sums + (size_t)(epoch & 1u) * 2 * kGpMaxGrid;
     double t = half(a, b2);
     if ((lane & 15) == 0) red[up][warp] = t;
     __syncthreads();
@@ -474,8 +476,8 @@ cfd_status grid_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, cons
   if (!fits) return CFD_OK;
   // published sums and z (zeroed: no flag set), r, p
   const size_t words = 4 * (size_t)kGpMaxGrid + (size_t)n;
-  uint4* ws = nullptr;
-  if (cudaMallocAsync((void**)&ws, words * sizeof(uint4) + 2 * (size_t)n * sizeof(double), ctx->stream) !=
+  ulonglong2* ws = nullptr;
+  if (cudaMallocAsync((void**)&ws, words * sizeof(ulonglong2) + 2 * (size_t)n * sizeof(double), ctx->stream) !=
       cudaSuccess) {
     cudaGetLastError();
     return CFD_OK;  // the multi-kernel solve reports an allocation that fails there too
@@ -485,7 +487,7 @@ cfd_status grid_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, cons
   A.r = reinterpret_cast<double*>(ws + words);
   A.p = A.r + n;
   cfd_status s = CFD_OK;
-  cudaError_t e = cudaMemsetAsync(ws, 0, words * sizeof(uint4), ctx->stream);
+  cudaError_t e = cudaMemsetAsync(ws, 0, words * sizeof(ulonglong2), ctx->stream);
   // two launches between looks at the state: one that finds the solve done returns at once
   while (e == cudaSuccess && s == CFD_OK) {
     for (int k = 0; k < 2 && s == CFD_OK; ++k) {
