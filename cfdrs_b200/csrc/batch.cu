@@ -777,21 +777,22 @@ cfd_status run_bucket(cfd_batch* bt, int bkt, int threads, int groups, cudaStrea
 // The device part of one batched solve: reset the queues, then one persistent
 // launch per bucket, each on a stream of its own between a fork and a join
 // (largest systems first).
-cfd_status enqueue_solve(cfd_batch* bt, int prec, const int* grid, const size_t* smem, cudaStream_t s,
-                         const cudaStream_t* branch, const cudaEvent_t* ev) {
+static_assert(kBuckets == cfd_context::kBranches + 1, "a branch for every bucket but one");
+cfd_status enqueue_solve(cfd_batch* bt, int prec, const int* grid, const size_t* smem, cudaStream_t s) {
+  const cfd_context* c = bt->ctx;
   CFD_TRY_CUDA(cudaMemsetAsync(bt->queues, 0, kBuckets * sizeof(unsigned), s));
-  CFD_TRY_CUDA(cudaEventRecord(ev[0], s));
+  CFD_TRY_CUDA(cudaEventRecord(c->branch_fork, s));
   for (int k = kBuckets - 1; k >= 0; --k) {
-    if (k > 0) CFD_TRY_CUDA(cudaStreamWaitEvent(branch[k], ev[0], 0));
-    cudaStream_t q = k > 0 ? branch[k] : s;
+    if (k > 0) CFD_TRY_CUDA(cudaStreamWaitEvent(c->branch[k - 1], c->branch_fork, 0));
+    cudaStream_t q = k > 0 ? c->branch[k - 1] : s;
     if (prec)
       CFD_TRY(launch_bucket<true>(bt, k, bt->threads[prec][k], bt->groups[prec][k], grid[k], smem[k], q));
     else
       CFD_TRY(launch_bucket<false>(bt, k, bt->threads[prec][k], bt->groups[prec][k], grid[k], smem[k], q));
   }
   for (int k = kBuckets - 1; k > 0; --k) {
-    CFD_TRY_CUDA(cudaEventRecord(ev[k], branch[k]));
-    CFD_TRY_CUDA(cudaStreamWaitEvent(s, ev[k], 0));
+    CFD_TRY_CUDA(cudaEventRecord(c->branch_join[k - 1], c->branch[k - 1]));
+    CFD_TRY_CUDA(cudaStreamWaitEvent(s, c->branch_join[k - 1], 0));
   }
   return CFD_OK;
 }
@@ -812,23 +813,10 @@ cfd_status capture_graph(cfd_batch* bt, int prec) {
   }
   // The buckets are parallel branches: a bucket's CTAs start where the larger
   // ones' queue has run dry.
-  struct Branches {
-    cudaStream_t s[kBuckets] = {};
-    cudaEvent_t e[kBuckets] = {};
-    ~Branches() {
-      for (int k = 0; k < kBuckets; ++k) {
-        if (e[k]) cudaEventDestroy(e[k]);
-        if (s[k]) cudaStreamDestroy(s[k]);
-      }
-    }
-  } br;
-  for (int k = 0; k < kBuckets; ++k) {
-    CFD_TRY_CUDA(cudaStreamCreateWithFlags(&br.s[k], cudaStreamNonBlocking));
-    CFD_TRY_CUDA(cudaEventCreateWithFlags(&br.e[k], cudaEventDisableTiming));
-  }
+  CFD_TRY(ensure_branches(bt->ctx));
   cudaGraph_t g = nullptr;
   CFD_TRY_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  cfd_status st = enqueue_solve(bt, prec, grid, smem, s, br.s, br.e);
+  cfd_status st = enqueue_solve(bt, prec, grid, smem, s);
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (st != CFD_OK) {
     if (g) cudaGraphDestroy(g);
@@ -1230,9 +1218,6 @@ cfd_status cfd_batch_destroy(cfd_batch* bt) {
                   (void*)bt->ls_pivot, (void*)bt->ls_plan_heads, (void*)bt->ls_plan_rounds,
                   (void*)bt->ls_plan_words, (void*)bt->ls_plan_init})
     if (p) cudaFree(p);
-  if (bt->ls_branch) cudaStreamDestroy(bt->ls_branch);
-  if (bt->ls_fork) cudaEventDestroy(bt->ls_fork);
-  if (bt->ls_join) cudaEventDestroy(bt->ls_join);
   if (bt->h_params) cudaFreeHost(bt->h_params);
   network_plan_free(bt->net);
   delete bt;

@@ -80,8 +80,6 @@ struct cfd_batch {
   int* ls_list = nullptr;
   double* ls_params = nullptr;
   unsigned* ls_queue = nullptr;
-  cudaStream_t ls_branch = nullptr;  // the second Krylov bucket, between fork and join
-  cudaEvent_t ls_fork = nullptr, ls_join = nullptr;
   double* ls_scratch = nullptr;
   size_t ls_scratch_elems = 0;
   int* ls_pivot = nullptr;   // per system: the dense fast path's pivot guard fired

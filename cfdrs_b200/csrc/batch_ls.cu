@@ -1545,9 +1545,7 @@ cfd_status ls_alloc(T** p, int64_t n) {
 // Per-system result arrays, the device lists and the parameter block, made
 // at the first cascade solve of a batch.
 cfd_status ls_prepare(cfd_batch* bt) {
-  if (!bt->ls_branch) CFD_TRY_CUDA(cudaStreamCreateWithFlags(&bt->ls_branch, cudaStreamNonBlocking));
-  if (!bt->ls_fork) CFD_TRY_CUDA(cudaEventCreateWithFlags(&bt->ls_fork, cudaEventDisableTiming));
-  if (!bt->ls_join) CFD_TRY_CUDA(cudaEventCreateWithFlags(&bt->ls_join, cudaEventDisableTiming));
+  CFD_TRY(ensure_branches(bt->ctx));
   if (bt->ls_path) return CFD_OK;
   CFD_TRY(ls_alloc(&bt->ls_method, bt->nsys));
   CFD_TRY(ls_alloc(&bt->ls_path, bt->nsys));
@@ -1873,15 +1871,16 @@ cfd_status cfd_batch_linear_system_solve(cfd_batch* bt, const cfd_ls_options* op
     // the buckets side by side: the smaller systems' CTAs start where the larger
     // ones' queue has run dry
     static_assert(kBuckets == 4, "one branch beside the solve's stream");
-    CFD_TRY_CUDA(cudaEventRecord(bt->ls_fork, s));
-    CFD_TRY_CUDA(cudaStreamWaitEvent(bt->ls_branch, bt->ls_fork, 0));
+    cudaStream_t branch = ctx->branch[0];
+    CFD_TRY_CUDA(cudaEventRecord(ctx->branch_fork, s));
+    CFD_TRY_CUDA(cudaStreamWaitEvent(branch, ctx->branch_fork, 0));
     cfd_status kst = CFD_OK;
     for (int k = kBuckets - 1; k >= 2 && kst == CFD_OK; --k) {
-      cudaStream_t q = k == kBuckets - 1 ? s : bt->ls_branch;
+      cudaStream_t q = k == kBuckets - 1 ? s : branch;
       kst = opt->precision ? ls_krylov_bucket<true>(bt, A, k, q) : ls_krylov_bucket<false>(bt, A, k, q);
     }
-    CFD_TRY_CUDA(cudaEventRecord(bt->ls_join, bt->ls_branch));
-    CFD_TRY_CUDA(cudaStreamWaitEvent(s, bt->ls_join, 0));
+    CFD_TRY_CUDA(cudaEventRecord(ctx->branch_join[0], branch));
+    CFD_TRY_CUDA(cudaStreamWaitEvent(s, ctx->branch_join[0], 0));
     CFD_TRY(kst);
     CFD_TRY_CUDA(cudaEventRecord(ph.e[2], s));
     std::vector<int> path(bt->nsys), method(bt->nsys), term(bt->nsys), iters(bt->nsys);

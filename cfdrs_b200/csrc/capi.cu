@@ -304,6 +304,16 @@ cfd_status check_device_flag(cfd_context* ctx) {
   return CFD_OK;
 }
 
+cfd_status ensure_branches(cfd_context* ctx) {
+  for (int k = 0; k < cfd_context::kBranches; ++k) {
+    if (!ctx->branch[k]) CFD_TRY_CUDA(cudaStreamCreateWithFlags(&ctx->branch[k], cudaStreamNonBlocking));
+    if (!ctx->branch_join[k])
+      CFD_TRY_CUDA(cudaEventCreateWithFlags(&ctx->branch_join[k], cudaEventDisableTiming));
+  }
+  if (!ctx->branch_fork) CFD_TRY_CUDA(cudaEventCreateWithFlags(&ctx->branch_fork, cudaEventDisableTiming));
+  return CFD_OK;
+}
+
 // Diagonal of A (FP64/FP32) and the DiagJacobi inverse: 1/a_ii, or 1 where
 // |a_ii| <= f64::EPSILON (linear_system.rs:286-295); a non-finite diagonal
 // entry makes the Jacobi preconditioner unavailable (linear_system.rs:281-285).
@@ -607,6 +617,11 @@ cfd_status cfd_context_destroy(cfd_context* ctx) {
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->ev_switch) cudaEventDestroy(ctx->ev_switch);
+  if (ctx->branch_fork) cudaEventDestroy(ctx->branch_fork);
+  for (int k = 0; k < cfd_context::kBranches; ++k) {
+    if (ctx->branch_join[k]) cudaEventDestroy(ctx->branch_join[k]);
+    if (ctx->branch[k]) cudaStreamDestroy(ctx->branch[k]);
+  }
   if (ctx->own) cudaStreamDestroy(ctx->own);
   delete ctx;
   return CFD_OK;

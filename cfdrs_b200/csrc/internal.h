@@ -309,6 +309,12 @@ struct cfd_context {
   cfd::DevState* h_state = nullptr;  // pinned mirror
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t ev_switch = nullptr;  // orders the old stream before the new one on a stream switch
+  // Parallel branches of the batched solves, between a fork and a join: made at the
+  // first batch of the context (streams and events made and destroyed at every new
+  // batch were 0.4 of the 0.8 ms of a small batch's first solve).
+  static constexpr int kBranches = 3;
+  cudaStream_t branch[kBranches] = {};
+  cudaEvent_t branch_fork = nullptr, branch_join[kBranches] = {};
   int* err = nullptr;    // set by a kernel whose bounded wait ran out
   int* h_err = nullptr;  // pinned mirror
   int num_sms = 148;
@@ -377,6 +383,7 @@ cfd_status allow_dynamic_smem(Kernel kern, int device) {
 }
 
 cfd_status ensure_partials(cfd_context* ctx, int blocks);
+cfd_status ensure_branches(cfd_context* ctx);
 // Reads the device error flag; a set flag (a bounded wait ran out) is reported
 // as CFD_ERR_TIMEOUT and the flag and reduction ticket are reset.
 cfd_status check_device_flag(cfd_context* ctx);
