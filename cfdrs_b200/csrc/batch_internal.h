@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "cfdgpu.h"
+#include "ls_plan.h"
 
 namespace cfd {
 
@@ -22,8 +23,6 @@ struct BatchParams {
 };
 
 struct NetworkPlanDev;  // network.cu
-struct LsPlanHead;      // ls_plan.h
-struct LsRound;
 
 // Checks a batch layout (offsets, row_ptr, local columns) without touching
 // any device state; see cfd_batch_create.
@@ -84,11 +83,16 @@ struct cfd_batch {
   size_t ls_scratch_elems = 0;
   int* ls_pivot = nullptr;   // per system: the dense fast path's pivot guard fired
   int64_t ls_pivoted = 0;    // systems handed to the pivoting dense solve, all calls
-  // Elimination plans (ls_plan.h), made from the pattern at the first direct
-  // solve; core sizes per system, -1: no plan.
+  // Elimination plans (ls_plan.h), a system's made from its pattern at its first
+  // direct solve: core sizes per system (kLsPlanUnknown, kLsPlanNone), heads and the
+  // slots of the stored entries as the device has them.
+  static constexpr int kLsPlanUnknown = -2, kLsPlanNone = -1;
   cfd::LsPlanHead* ls_plan_heads = nullptr;
   cfd::LsRound* ls_plan_rounds = nullptr;
   uint16_t* ls_plan_words = nullptr;
   uint16_t* ls_plan_init = nullptr;
+  size_t ls_plan_words_room = 0, ls_plan_words_used = 0, ls_plan_rounds_room = 0, ls_plan_rounds_used = 0;
   std::vector<int> ls_plan_core;
+  std::vector<cfd::LsPlanHead> ls_plan_host;
+  std::vector<uint16_t> ls_plan_slots;
 };

@@ -24,6 +24,7 @@
 // a dense core where the pattern has such an order (k_ls_sparse, ls_plan.h), the
 // others, and those that need row exchanges, by a second dense launch.
 #include <cuda_runtime.h>
+#include <omp.h>
 
 #include <algorithm>
 #include <cfloat>
@@ -35,7 +36,6 @@
 #include "batch_internal.h"
 #include "internal.h"
 #include "kernels.cuh"
-#include "ls_plan.h"
 
 namespace cfd {
 namespace {
@@ -1622,71 +1622,106 @@ cfd_status ls_dense_launch(cfd_batch* bt, const LsArgs& A, const std::vector<int
   return CFD_OK;
 }
 
-// The elimination plans, made from the batch's pattern at its first direct solve.
-cfd_status ls_ensure_plans(cfd_batch* bt, cudaStream_t s) {
-  if (bt->ls_plan_heads) return CFD_OK;
+// A device array that grows at its end, what it holds kept.
+template <typename T>
+cfd_status ls_grow(T** p, size_t* room, size_t used, size_t need, cudaStream_t s) {
+  if (need <= *room) return CFD_OK;
+  const size_t to = std::max(need, *room + *room / 2);
+  T* q = nullptr;
+  CFD_TRY(ls_alloc(&q, (int64_t)to));
+  if (used > 0) {
+    cudaError_t e = cudaMemcpyAsync(q, *p, used * sizeof(T), cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+      cudaFree(q);
+      CFD_TRY_CUDA(e);
+    }
+  }
+  if (*p) cudaFree(*p);
+  *p = q;
+  *room = to;
+  return CFD_OK;
+}
+
+// Elimination plans of the systems in `list` that have not been looked at: a batch
+// makes a system's plan when it first solves it directly, for a Krylov solve that
+// is kept needs none. Each host thread writes its plans one after another, and the
+// threads' parts go to the device one behind the other (which part a plan is in does
+// not matter to it).
+cfd_status ls_ensure_plans(cfd_batch* bt, const std::vector<int>& list, cudaStream_t s) {
+  if (bt->ls_plan_core.empty()) {
+    bt->ls_plan_core.assign(bt->nsys, cfd_batch::kLsPlanUnknown);
+    bt->ls_plan_host.assign(bt->nsys, LsPlanHead{});
+    bt->ls_plan_slots.assign(bt->nnz, 0);
+  }
+  std::vector<int> todo;
+  for (int sy : list)
+    if (bt->ls_plan_core[sy] == cfd_batch::kLsPlanUnknown) todo.push_back(sy);
+  if (todo.empty()) return CFD_OK;
   std::vector<int> rp(bt->rows + 1), col(bt->nnz);
   CFD_TRY_CUDA(cudaMemcpyAsync(rp.data(), bt->rp, rp.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
   CFD_TRY_CUDA(cudaMemcpyAsync(col.data(), bt->col, col.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
   CFD_TRY_CUDA(cudaStreamSynchronize(s));
-  const int todo = bt->nsys;
-  std::vector<LsPlanOne> plans(todo);
+  // a thread for every 2000 rows (about a millisecond of one)
+  int64_t rows = 0;
+  for (int sy : todo) rows += bt->h_sys_row[sy + 1] - bt->h_sys_row[sy];
+  const int count = (int)todo.size(), threads = (int)std::min<int64_t>(omp_get_max_threads(), 1 + rows / 2000);
+  std::vector<LsPlanSet> sets(threads);
+  std::vector<int> part(count);
   int failed = 0;
-#pragma omp parallel for schedule(dynamic, 4)
-  for (int q = 0; q < todo; ++q) {
-    try {  // no exception leaves the parallel region
-      const int sy = bt->h_order[q], r0 = bt->h_sys_row[sy];
-      ls_plan_build(bt->h_sys_row[sy + 1] - r0, rp.data() + r0, col.data(), plans[q]);
-    } catch (...) {
+#pragma omp parallel num_threads(threads)
+  {
+    LsPlanWork work;
+    const int me = omp_get_thread_num();
+#pragma omp for schedule(dynamic, 4)
+    for (int q = 0; q < count; ++q) {
+      try {  // no exception leaves the parallel region
+        const int sy = todo[q], r0 = bt->h_sys_row[sy];
+        part[q] = me;
+        ls_plan_build(bt->h_sys_row[sy + 1] - r0, rp.data() + r0, col.data(), work, sets[me],
+                      bt->ls_plan_slots.data() + rp[r0], bt->ls_plan_host[sy]);
+      } catch (...) {
 #pragma omp atomic write
-      failed = 1;
+        failed = 1;
+      }
     }
   }
   if (failed) {
     set_error("cfd_batch_linear_system_solve: host memory for the elimination plans");
     return CFD_ERR_ALLOC;
   }
-  std::vector<LsPlanHead> heads(bt->nsys);
-  std::vector<LsRound> rounds;
-  std::vector<uint16_t> init(bt->nnz, 0), words;
-  bt->ls_plan_core.assign(bt->nsys, -1);
-  for (int q = 0; q < todo; ++q) {
-    const int sy = bt->h_order[q];
-    LsPlanOne& P = plans[q];
-    if (!P.head.ok) continue;
-    P.head.words = (int64_t)words.size();
-    P.head.round0 = (int32_t)rounds.size();
-    words.insert(words.end(), P.words.begin(), P.words.end());
-    rounds.insert(rounds.end(), P.rounds.begin(), P.rounds.end());
-    std::copy(P.init.begin(), P.init.end(), init.begin() + rp[bt->h_sys_row[sy]]);
-    heads[sy] = P.head;
-    bt->ls_plan_core[sy] = P.head.core;
-    P = LsPlanOne{};
+  std::vector<size_t> word0(threads), round0(threads);
+  size_t words = bt->ls_plan_words_used, rounds = bt->ls_plan_rounds_used;
+  for (int t = 0; t < threads; ++t) {
+    word0[t] = words;
+    round0[t] = rounds;
+    words += sets[t].words.size();
+    rounds += sets[t].rounds.size();
   }
-  cfd_status st = ls_alloc(&bt->ls_plan_words, (int64_t)words.size());
-  if (st == CFD_OK) st = ls_alloc(&bt->ls_plan_init, (int64_t)init.size());
-  if (st == CFD_OK) st = ls_alloc(&bt->ls_plan_rounds, (int64_t)rounds.size());
-  LsPlanHead* dev = nullptr;
-  if (st == CFD_OK) st = ls_alloc(&dev, (int64_t)heads.size());
-  auto up = [&](void* d, const void* h, size_t bytes) {
-    if (st == CFD_OK && bytes > 0 && cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess) {
-      set_error("cfd_batch_linear_system_solve: upload of the elimination plans failed");
-      st = CFD_ERR_CUDA;
-    }
-  };
-  up(bt->ls_plan_words, words.data(), words.size() * sizeof(uint16_t));
-  up(bt->ls_plan_init, init.data(), init.size() * sizeof(uint16_t));
-  up(bt->ls_plan_rounds, rounds.data(), rounds.size() * sizeof(LsRound));
-  up(dev, heads.data(), heads.size() * sizeof(LsPlanHead));
-  if (st == CFD_OK && cudaStreamSynchronize(s) != cudaSuccess) st = CFD_ERR_CUDA;
-  if (st != CFD_OK) {
-    for (void* p : {(void*)bt->ls_plan_words, (void*)bt->ls_plan_init, (void*)bt->ls_plan_rounds, (void*)dev})
-      if (p) cudaFree(p);
-    bt->ls_plan_words = bt->ls_plan_init = nullptr;
-    bt->ls_plan_rounds = nullptr;
-    return st;
+  CFD_TRY(ls_grow(&bt->ls_plan_words, &bt->ls_plan_words_room, bt->ls_plan_words_used, words, s));
+  CFD_TRY(ls_grow(&bt->ls_plan_rounds, &bt->ls_plan_rounds_room, bt->ls_plan_rounds_used, rounds, s));
+  if (!bt->ls_plan_init) CFD_TRY(ls_alloc(&bt->ls_plan_init, bt->nnz));
+  if (!bt->ls_plan_heads) CFD_TRY(ls_alloc(&bt->ls_plan_heads, bt->nsys));
+  for (int t = 0; t < threads; ++t) {
+    CFD_TRY_CUDA(cudaMemcpyAsync(bt->ls_plan_words + word0[t], sets[t].words.data(),
+                                 sets[t].words.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
+    CFD_TRY_CUDA(cudaMemcpyAsync(bt->ls_plan_rounds + round0[t], sets[t].rounds.data(),
+                                 sets[t].rounds.size() * sizeof(LsRound), cudaMemcpyHostToDevice, s));
   }
-  bt->ls_plan_heads = dev;
+  std::vector<LsPlanHead>& heads = bt->ls_plan_host;
+  for (int q = 0; q < count; ++q) {
+    heads[todo[q]].words += (int64_t)word0[part[q]];
+    heads[todo[q]].round0 += (int32_t)round0[part[q]];
+  }
+  CFD_TRY_CUDA(cudaMemcpyAsync(bt->ls_plan_init, bt->ls_plan_slots.data(), bt->nnz * sizeof(uint16_t),
+                               cudaMemcpyHostToDevice, s));
+  CFD_TRY_CUDA(cudaMemcpyAsync(bt->ls_plan_heads, heads.data(), heads.size() * sizeof(LsPlanHead),
+                               cudaMemcpyHostToDevice, s));
+  CFD_TRY_CUDA(cudaStreamSynchronize(s));
+  // only now: a call that failed on the way looks at these systems again
+  bt->ls_plan_words_used = words;
+  bt->ls_plan_rounds_used = rounds;
+  for (int sy : todo) bt->ls_plan_core[sy] = heads[sy].ok ? heads[sy].core : cfd_batch::kLsPlanNone;
   return CFD_OK;
 }
 
@@ -1696,11 +1731,11 @@ cfd_status ls_ensure_plans(cfd_batch* bt, cudaStream_t s) {
 cfd_status ls_direct_launch(cfd_batch* bt, const LsArgs& A, const std::vector<int>& list, bool direct,
                             cudaStream_t s) {
   if (list.empty()) return CFD_OK;
-  CFD_TRY(ls_ensure_plans(bt, s));
+  CFD_TRY(ls_ensure_plans(bt, list, s));
   std::vector<int> sparse, dense;
   int cmax = 0;
   for (int sy : list) {
-    if (bt->ls_plan_core[sy] < 0) {
+    if (bt->ls_plan_core[sy] == cfd_batch::kLsPlanNone) {
       dense.push_back(sy);
       continue;
     }

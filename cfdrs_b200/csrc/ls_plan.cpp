@@ -8,79 +8,77 @@ namespace {
 
 constexpr int kNone = -1;
 
-// A neighbour j of node i: the slots of entries (i, j) and (j, i).
-struct Nb {
-  int node, out, in;
-};
+using Nb = LsPlanWork::Nb;
 
-// Neighbour lists in one array: a list that outgrows its place moves to the end.
+// The neighbour lists: a list that outgrows its place moves to the end.
 class Lists {
  public:
-  Lists(int n, int total) : at_(n, 0), len_(n, 0), room_(n, 0) { pool_.reserve((size_t)4 * total + 64); }
-  int size(int i) const { return len_[i]; }
-  Nb* begin(int i) { return pool_.data() + at_[i]; }
-  Nb* end(int i) { return begin(i) + len_[i]; }
+  Lists(LsPlanWork& w, int n, int total) : w_(w) {
+    w_.at.assign(n, 0);
+    w_.len.assign(n, 0);
+    w_.room.assign(n, 0);
+    w_.pool.clear();
+    w_.pool.reserve((size_t)4 * total + 64);
+  }
+  int size(int i) const { return w_.len[i]; }
+  Nb* begin(int i) { return w_.pool.data() + w_.at[i]; }
+  Nb* end(int i) { return begin(i) + w_.len[i]; }
   Nb* find(int i, int node) {
     for (Nb* q = begin(i); q != end(i); ++q)
       if (q->node == node) return q;
     return nullptr;
   }
   void push(int i, const Nb& b) {
-    if (len_[i] == room_[i]) {
-      const int room = room_[i] ? 2 * room_[i] : 4;
-      const size_t to = pool_.size();
-      pool_.resize(to + room);
-      std::copy(pool_.begin() + at_[i], pool_.begin() + at_[i] + len_[i], pool_.begin() + to);
-      at_[i] = to;
-      room_[i] = room;
+    if (w_.len[i] == w_.room[i]) {
+      const int room = w_.room[i] ? 2 * w_.room[i] : 4;
+      const size_t to = w_.pool.size();
+      w_.pool.resize(to + room);
+      std::copy(w_.pool.begin() + w_.at[i], w_.pool.begin() + w_.at[i] + w_.len[i], w_.pool.begin() + to);
+      w_.at[i] = to;
+      w_.room[i] = room;
     }
-    begin(i)[len_[i]++] = b;
+    begin(i)[w_.len[i]++] = b;
   }
   void drop(int i, int node) {  // keeps the order of the others
     Nb* q = find(i, node);
     std::copy(q + 1, end(i), q);
-    --len_[i];
+    --w_.len[i];
   }
 
  private:
-  std::vector<Nb> pool_;
-  std::vector<size_t> at_;
-  std::vector<int> len_, room_;
-};
-
-struct Update {
-  int target, i, j;
+  LsPlanWork& w_;
 };
 
 }  // namespace
 
-void ls_plan_build(int n, const int* rp, const int* col, LsPlanOne& out) {
-  out = LsPlanOne{};
+bool ls_plan_build(int n, const int* rp, const int* col, LsPlanWork& work, LsPlanSet& set, uint16_t* init,
+                   LsPlanHead& head) {
+  head = LsPlanHead{};
   const int k0 = rp[0], nnz = rp[n] - k0;
-  std::vector<int> diag(n, kNone);
-  int slots = 0;
-  out.init.resize(nnz);
   // A pattern this wide has no sparse order worth writing out.
-  if (nnz > 8 * n + 64) return;
-  Lists adj(n, nnz);
+  if (nnz > 8 * n + 64) return false;
+  int slots = 0;
+  auto& diag = work.diag;
+  diag.assign(n, kNone);
+  Lists adj(work, n, nnz);
   for (int i = 0; i < n; ++i)
     for (int e = rp[i]; e < rp[i + 1]; ++e) {
       const int j = col[e];
-      int* s;
-      if (j == i) {
-        s = &diag[i];
-      } else {
-        if (!adj.find(i, j)) {
-          adj.push(i, {j, kNone, kNone});
+      int* s = &diag[i];
+      if (j != i) {
+        Nb* q = adj.find(i, j);
+        if (!q) {
           adj.push(j, {i, kNone, kNone});
+          adj.push(i, {j, kNone, kNone});
+          q = adj.end(i) - 1;
         }
-        s = &adj.find(i, j)->out;
+        s = &q->out;
       }
       if (*s == kNone) {  // a repeated entry adds into the first one's slot
         *s = slots++;
         if (j != i) adj.find(j, i)->in = *s;
       }
-      out.init[e - k0] = (uint16_t)*s;
+      init[e - k0] = (uint16_t)*s;
     }
   auto fill = [&](int i, int j) -> int {  // slot (i, j), the pair made where the pattern lacks it
     Nb* q = adj.find(i, j);
@@ -101,137 +99,164 @@ void ls_plan_build(int n, const int* rp, const int* col, LsPlanOne& out) {
   }
   // Right-hand-side slots are numbered after the fill: bslot(i) = ~i until then.
   auto bslot = [](int i) { return ~i; };
-  struct Round {
-    std::vector<std::pair<int, int>> div;
-    std::vector<Update> upd;
-    std::vector<int> nodes;
-    std::vector<Nb> nbs;       // the nodes' neighbours when they go
-    std::vector<int> nb_end;
-  };
-  std::vector<Round> rounds;
-  std::vector<char> alive(n, 1);
-  std::vector<int> blocked(n, -1);
-  int left = n;
-  for (int r = 0; left > 0; ++r) {
+  auto& div = work.div;
+  auto& upd = work.upd;
+  auto &nodes = work.nodes, &live = work.live, &blocked = work.blocked;
+  auto& nbs = work.nbs;  // the nodes' neighbours when they go
+  auto& nb_end = work.nb_end;
+  auto& rounds = work.rounds;
+  auto& alive = work.alive;
+  div.clear();
+  upd.clear();
+  nodes.clear();
+  nbs.clear();
+  nb_end.clear();
+  rounds.clear();
+  live.resize(n);
+  for (int i = 0; i < n; ++i) live[i] = i;
+  blocked.assign(n, -1);
+  alive.assign(n, 1);
+  for (int r = 0; !live.empty(); ++r) {
     int lo = n;
-    for (int i = 0; i < n; ++i)
-      if (alive[i]) lo = std::min(lo, adj.size(i));
+    for (auto& q : work.by_degree) q.clear();
+    for (int v : live) {
+      const int d = adj.size(v);
+      lo = std::min(lo, d);
+      if (d <= kLsPlanDegree) work.by_degree[d].push_back(v);
+    }
     if (lo > kLsPlanDegree) break;
-    const int cap = std::max(2, lo);
-    Round R;
-    for (int deg = 0; deg <= cap; ++deg)
-      for (int v = 0; v < n; ++v) {
-        if (!alive[v] || adj.size(v) != deg || blocked[v] == r) continue;
-        R.nodes.push_back(v);
+    const LsPlanWork::Round R{div.size(), upd.size(), nodes.size(), nbs.size()};
+    for (int deg = 0; deg <= std::max(2, lo); ++deg)
+      for (int v : work.by_degree[deg]) {
+        if (blocked[v] == r) continue;
+        nodes.push_back(v);
         blocked[v] = r;
         for (Nb* q = adj.begin(v); q != adj.end(v); ++q) blocked[q->node] = r;
       }
-    for (int v : R.nodes) {
-      const size_t b = R.nbs.size();
-      R.nbs.insert(R.nbs.end(), adj.begin(v), adj.end(v));
-      R.nb_end.push_back((int)R.nbs.size());
-      for (size_t a = b; a < R.nbs.size(); ++a) {
-        const Nb u = R.nbs[a];
-        R.div.push_back({u.in, diag[v]});
-        R.upd.push_back({bslot(u.node), u.in, bslot(v)});
-        for (size_t c = b; c < R.nbs.size(); ++c)
-          R.upd.push_back({a == c ? diag[u.node] : fill(u.node, R.nbs[c].node), u.in, R.nbs[c].out});
+    for (size_t q = R.node; q < nodes.size(); ++q) {
+      const int v = nodes[q];
+      const size_t b = nbs.size();
+      nbs.insert(nbs.end(), adj.begin(v), adj.end(v));
+      nb_end.push_back(nbs.size());
+      for (size_t a = b; a < nbs.size(); ++a) {
+        const Nb u = nbs[a];
+        div.push_back({u.in, diag[v]});
+        upd.push_back({bslot(u.node), u.in, bslot(v), kNone});
+        for (size_t c = b; c < nbs.size(); ++c)
+          upd.push_back({a == c ? diag[u.node] : fill(u.node, nbs[c].node), u.in, nbs[c].out, kNone});
       }
     }
-    for (size_t q = 0, a = 0; q < R.nodes.size(); ++q) {
-      for (; a < (size_t)R.nb_end[q]; ++a) adj.drop(R.nbs[a].node, R.nodes[q]);
-      alive[R.nodes[q]] = 0;
-      --left;
+    for (size_t q = R.node, a = R.nb; q < nodes.size(); ++q) {
+      for (; a < nb_end[q]; ++a) adj.drop(nbs[a].node, nodes[q]);
+      alive[nodes[q]] = 0;
     }
-    rounds.push_back(std::move(R));
-    if (slots + n > kLsPlanMaxSlots) return;
+    live.erase(std::remove_if(live.begin(), live.end(), [&](int v) { return !alive[v]; }), live.end());
+    rounds.push_back(R);
+    if (slots + n > kLsPlanMaxSlots) return false;
   }
   const int b0 = slots;
   slots += n;
-  if (slots > kLsPlanMaxSlots || 2 * left > n) return;
-  auto slot = [&](int s) { return (uint16_t)(s < 0 ? b0 + ~s : s); };
-  auto& w = out.words;
-  std::vector<int> count(slots + 1);
-  std::vector<Update> sorted;
-  for (Round& R : rounds) {
-    LsRound d{};
-    d.at_l = (int32_t)w.size();
-    d.nl = (int32_t)R.div.size();
-    for (auto& q : R.div) {
-      w.push_back(slot(q.first));
-      w.push_back(slot(q.second));
-    }
+  if (slots > kLsPlanMaxSlots || 2 * (int)live.size() > n) return false;
+  auto slot = [&](int s) { return s < 0 ? b0 + ~s : s; };
+  for (size_t q = 0; q < rounds.size(); ++q)
+    if ((q + 1 == rounds.size() ? upd.size() : rounds[q + 1].upd) - rounds[q].upd > 65535) return false;
+  auto& w = set.words;  // offsets are from this system's first word
+  head.words = (int64_t)w.size();
+  head.round0 = (int32_t)set.rounds.size();
+  const size_t w0 = w.size();
+  auto &first = work.first, &last = work.last, &order = work.order;
+  first.assign(slots, kNone);
+  last.resize(slots);
+  for (size_t q = 0; q < rounds.size(); ++q) {
+    const LsPlanWork::Round& R = rounds[q];
+    const bool end = q + 1 == rounds.size();
+    const size_t div_e = end ? div.size() : rounds[q + 1].div, upd_e = end ? upd.size() : rounds[q + 1].upd;
+    const size_t node_e = end ? nodes.size() : rounds[q + 1].node, nb_e = end ? nbs.size() : rounds[q + 1].nb;
     // by target, the order within a target kept
-    std::fill(count.begin(), count.end(), 0);
-    for (Update& q : R.upd) {
-      q.target = slot(q.target);
-      count[q.target + 1]++;
-    }
-    for (int k = 0; k < slots; ++k) count[k + 1] += count[k];
-    sorted.resize(R.upd.size());
-    for (const Update& q : R.upd) sorted[count[q.target]++] = q;
-    R.upd.swap(sorted);
-    std::vector<uint16_t> pairs;
-    d.at_t = (int32_t)w.size();
-    for (size_t q = 0; q < R.upd.size();) {
-      const size_t first = q;
-      while (q < R.upd.size() && R.upd[q].target == R.upd[first].target) {
-        pairs.push_back(slot(R.upd[q].i));
-        pairs.push_back(slot(R.upd[q].j));
-        ++q;
+    order.clear();
+    for (size_t u = R.upd; u < upd_e; ++u) {
+      const int t = slot(upd[u].target);
+      if (first[t] == kNone) {
+        first[t] = (int)u;
+        order.push_back(t);
+      } else {
+        upd[last[t]].next = (int)u;
       }
-      w.push_back((uint16_t)R.upd[first].target);
-      w.push_back((uint16_t)first);
-      w.push_back((uint16_t)(q - first));
-      d.nt++;
+      last[t] = (int)u;
     }
-    if (R.upd.size() > 65535) return;
-    d.pairs = (int32_t)w.size();
-    w.insert(w.end(), pairs.begin(), pairs.end());
-    pairs.clear();
-    d.at_x = (int32_t)w.size();
-    d.nx = (int32_t)R.nodes.size();
-    for (size_t q = 0; q < R.nodes.size(); ++q) {
-      w.push_back(slot(bslot(R.nodes[q])));
-      w.push_back(slot(diag[R.nodes[q]]));
-      w.push_back((uint16_t)(pairs.size() / 2));
-      const int b = q ? R.nb_end[q - 1] : 0;
-      w.push_back((uint16_t)(R.nb_end[q] - b));
-      for (int a = b; a < R.nb_end[q]; ++a) {
-        pairs.push_back(slot(R.nbs[a].out));
-        pairs.push_back(slot(bslot(R.nbs[a].node)));
+    LsRound d{};
+    d.nl = (int32_t)(div_e - R.div);
+    d.nt = (int32_t)order.size();
+    d.nx = (int32_t)(node_e - R.node);
+    d.at_l = (int32_t)(w.size() - w0);
+    d.at_t = d.at_l + 2 * d.nl;
+    d.pairs = d.at_t + 3 * d.nt;
+    d.at_x = d.pairs + 2 * (int32_t)(upd_e - R.upd);
+    d.xpairs = d.at_x + 4 * d.nx;
+    w.resize(w0 + (size_t)d.xpairs + 2 * (nb_e - R.nb));
+    uint16_t* const words = w.data() + w0;
+    uint16_t* o = words + d.at_l;
+    for (size_t k = R.div; k < div_e; ++k) {
+      *o++ = (uint16_t)div[k].first;
+      *o++ = (uint16_t)div[k].second;
+    }
+    uint16_t* p = words + d.pairs;
+    int at = 0;
+    for (int t : order) {
+      int count = 0;
+      for (int u = first[t]; u != kNone; u = upd[u].next, ++count) {
+        *p++ = (uint16_t)slot(upd[u].i);
+        *p++ = (uint16_t)slot(upd[u].j);
+      }
+      first[t] = kNone;
+      *o++ = (uint16_t)t;
+      *o++ = (uint16_t)at;
+      *o++ = (uint16_t)count;
+      at += count;
+    }
+    o = words + d.at_x;
+    p = words + d.xpairs;
+    size_t a = R.nb;
+    at = 0;
+    for (size_t k = R.node; k < node_e; ++k) {
+      *o++ = (uint16_t)slot(bslot(nodes[k]));
+      *o++ = (uint16_t)diag[nodes[k]];
+      *o++ = (uint16_t)at;
+      *o++ = (uint16_t)(nb_end[k] - a);
+      at += (int)(nb_end[k] - a);
+      for (; a < nb_end[k]; ++a) {
+        *p++ = (uint16_t)nbs[a].out;
+        *p++ = (uint16_t)slot(bslot(nbs[a].node));
       }
     }
-    d.xpairs = (int32_t)w.size();
-    w.insert(w.end(), pairs.begin(), pairs.end());
-    out.rounds.push_back(d);
+    set.rounds.push_back(d);
   }
-  std::vector<int> place(n, kNone);
+  auto& place = work.place;
+  place.assign(n, kNone);
   int core = 0;
-  out.head.at_core = (int32_t)w.size();
-  for (int i = 0; i < n; ++i)
-    if (alive[i]) {
-      place[i] = core++;
-      w.push_back((uint16_t)i);
-    }
-  out.head.at_entries = (int32_t)w.size();
-  for (int i = 0; i < n; ++i) {
-    if (!alive[i]) continue;
-    w.push_back(slot(diag[i]));
+  head.at_core = (int32_t)(w.size() - w0);
+  for (int i : live) {
+    place[i] = core++;
+    w.push_back((uint16_t)i);
+  }
+  head.at_entries = (int32_t)(w.size() - w0);
+  for (int i : live) {
+    w.push_back((uint16_t)diag[i]);
     w.push_back((uint16_t)place[i]);
     w.push_back((uint16_t)place[i]);
     for (Nb* u = adj.begin(i); u != adj.end(i); ++u) {
-      w.push_back(slot(u->out));
+      w.push_back((uint16_t)u->out);
       w.push_back((uint16_t)place[i]);
       w.push_back((uint16_t)place[u->node]);
     }
   }
-  out.head.entries = (int32_t)(w.size() - out.head.at_entries) / 3;
-  out.head.core = core;
-  out.head.slots = slots;
-  out.head.b0 = b0;
-  out.head.rounds = (int32_t)out.rounds.size();
-  out.head.ok = 1;
+  head.entries = (int32_t)((w.size() - w0 - head.at_entries) / 3);
+  head.core = core;
+  head.slots = slots;
+  head.b0 = b0;
+  head.rounds = (int32_t)rounds.size();
+  head.ok = 1;
+  return true;
 }
 
 }  // namespace cfd

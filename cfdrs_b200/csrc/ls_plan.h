@@ -15,6 +15,7 @@
 #pragma once
 
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 namespace cfd {
@@ -40,16 +41,42 @@ struct LsPlanHead {
   int32_t entries, at_entries;  // core entries: triples (slot, row, col)
   int32_t pad;
   int64_t words;          // this system's first word
-  int64_t init;           // slot of every stored entry, first word (the batch's entry order)
 };
 
-// The plan of one square pattern (rows rp[0..n], local columns); words and
-// rounds are appended, head.words / head.init left to the caller.
-struct LsPlanOne {
-  LsPlanHead head{};
-  std::vector<uint16_t> words, init;
+// Plans one after another.
+struct LsPlanSet {
+  std::vector<uint16_t> words;
   std::vector<LsRound> rounds;
 };
-void ls_plan_build(int n, const int* rp, const int* col, LsPlanOne& out);
+
+// Scratch of ls_plan_build, kept from one system to the next: with arrays of their
+// own for every system the builder spent half its time in the allocator.
+struct LsPlanWork {
+  struct Nb {  // a neighbour: its node, the slots of the entries to and from it
+    int node, out, in;
+  };
+  struct Update {  // v[target] -= v[i] v[j]; next: the target's next update of its round, -1 the last
+    int target, i, j, next;
+  };
+  struct Round {  // where a round's part of the arrays below begins
+    size_t div, upd, node, nb;
+  };
+  std::vector<Nb> pool;  // neighbour lists in one array
+  std::vector<size_t> at;
+  std::vector<int> len, room;
+  std::vector<int> diag, live, blocked, by_degree[kLsPlanDegree + 1], nodes, first, last, order, place;
+  std::vector<char> alive;
+  std::vector<std::pair<int, int>> div;
+  std::vector<Update> upd;
+  std::vector<Nb> nbs;
+  std::vector<size_t> nb_end;
+  std::vector<Round> rounds;
+};
+
+// The plan of one square pattern (rows rp[0..n], local columns), appended to the
+// set; init takes the slot of every stored entry. False where the pattern has none
+// (the set is as it was).
+bool ls_plan_build(int n, const int* rp, const int* col, LsPlanWork& work, LsPlanSet& set, uint16_t* init,
+                   LsPlanHead& head);
 
 }  // namespace cfd
