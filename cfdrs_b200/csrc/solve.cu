@@ -11,6 +11,7 @@
 #include <type_traits>
 
 #include "amg_device.h"
+#include "gmres_look.h"
 #include "internal.h"
 #include "simple.h"
 #include "kernels.cuh"
@@ -1304,12 +1305,6 @@ int gmres_width(int64_t requested) {
   return w;
 }
 
-// Steps until a residual that falls by `rate` a step passes the threshold.
-static double gmres_steps_left(double rn, const DevState& h, double rate) {
-  if (!(h.threshold > 0.0) || !(rn > h.threshold)) return 1.0;
-  return std::max(1.0, std::ceil(std::log(h.threshold / rn) / std::log(rate)));
-}
-
 // Restarted GMRES(m) with right preconditioning. Expects the state's start
 // (rnorm0, threshold, done, iter) set, r = b - A x and b the right-hand side.
 // The host polls at the end of a restart cycle and where the residual's rate says
@@ -1369,11 +1364,10 @@ static cfd_status gmres_loop(Launcher& lc, cfd_csr* a, cfd_amg* amg, KrylovBufs<
   // residual's rate says the cycle should end, and stops launching once it has.
   // A restart of 32 that converged in 17 steps ran 15 for nothing, 2.75 ms against
   // 2.02 ms on the 11^3 Stokes system. A rate that reaches past the restart costs
-  // no look.
+  // no look, nor does a threshold of zero (a run to a fixed budget) after the first.
   double rate = 0.0, rn_cycle = 0.0;
   for (;;) {
-    int look = 8;
-    if (cycles > 0) look = rate > 0.0 && rate < 1.0 ? (int)std::min(1e6, gmres_steps_left(rn_cycle, *pl.host, rate)) : m;
+    int look = cycles > 0 ? gmres_next_look(0, m, rn_cycle, pl.host->threshold, rate) : 8;
     int last_look = 0;
     double last_rn = rn_cycle;
     // cycle start: beta = ||r||, v_0 = r / beta
@@ -1408,7 +1402,7 @@ static cfd_status gmres_loop(Launcher& lc, cfd_csr* a, cfd_amg* amg, KrylovBufs<
         rate = from > 0.0 ? std::pow(h.rnorm / from, 1.0 / (double)(j + 1 - last_look)) : 0.0;
         last_look = j + 1;
         last_rn = h.rnorm;
-        look = rate > 0.0 && rate < 1.0 ? j + 1 + (int)std::min(1e6, gmres_steps_left(h.rnorm, h, rate)) : m;
+        look = gmres_next_look(j + 1, m, h.rnorm, h.threshold, rate);
       }
     }
     // x += M^-1 (V y); r = b - A x; the true residual decides
