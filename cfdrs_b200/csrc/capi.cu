@@ -314,9 +314,6 @@ cfd_status ensure_branches(cfd_context* ctx) {
   return CFD_OK;
 }
 
-// Diagonal of A (FP64/FP32) and the DiagJacobi inverse: 1/a_ii, or 1 where
-// |a_ii| <= f64::EPSILON (linear_system.rs:286-295); a non-finite diagonal
-// entry makes the Jacobi preconditioner unavailable (linear_system.rs:281-285).
 cfd_status csr_sync_host(cfd_csr* a) {
   if (!a->host_stale) return CFD_OK;
   cudaStream_t s = a->ctx->stream;
@@ -326,6 +323,9 @@ cfd_status csr_sync_host(cfd_csr* a) {
   return CFD_OK;
 }
 
+// Diagonal of A (FP64/FP32) and the DiagJacobi inverse: 1/a_ii, or 1 where
+// |a_ii| <= f64::EPSILON (linear_system.rs:286-295); a non-finite diagonal
+// entry makes the Jacobi preconditioner unavailable (linear_system.rs:281-285).
 cfd_status ensure_diagonals(cfd_csr* a) {
   if (a->diag64) return CFD_OK;
   CFD_TRY(csr_sync_host(a));

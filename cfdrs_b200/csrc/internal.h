@@ -240,7 +240,9 @@ bool check_diagonal(const HostCsr& h, const HostDiagonal& D, const double* x, st
 // setting, with CFD_PATH_AUTO resolved to RECORD for FP32 and X_STAGED for
 // FP64 one-thread rows (SPLIT for other FP64 matrices), as measured fastest on
 // the 256^3 AMG hierarchy, and ineligible pipelines stepped down. CFD_PATH_TIMED
-// is returned as is (the launcher times the pipelines first).
+// is returned as is (the launcher times the pipelines first). In place of the
+// pipeline that AUTO stands for, other than DIAGONAL, an operator small enough runs
+// the direct kernel (Launcher::direct_fits), which has no path value.
 inline int spmv_path(const DevMat& m, int p) {
   int path = m.path[p];
   if (path == CFD_PATH_TIMED) return path;

@@ -865,9 +865,9 @@ __global__ void __launch_bounds__(kPipeThreads, PipeLayout<VT, CODES>::kMinBlock
 // ---------------------------------------------------------------------------
 // Direct kernel for operators that sit in L2 (the coarse levels and their
 // transfers, small systems): no staging, every row group reads its row offsets,
-// entries and x from global memory, kDirectBatch entries a thread at a time
-// without branches (slots past the row's end repeat its last entry with zero
-// factors). What bounds such an operator is the chain of dependent latencies of
+// entries and x from global memory, kDirectBatch entries a thread at a time, their
+// loads without branches (slots past the row's end load its last entry again and are
+// left out of the sum). What bounds such an operator is the chain of dependent latencies of
 // one launch; here it is three loads (offsets, entries, x), and the done flag is
 // read beside them and tested before anything is written, where the bulk-copy
 // pipelines add barrier set-up, descriptors and the copy itself. Row groups and

@@ -116,7 +116,8 @@ typedef struct {
   int32_t threads_per_row;
   int32_t max_windows;       /* cfd_layout_check only */
   int64_t staged_x_entries;  /* cfd_layout_check only: x entries staged over all blocks */
-  int32_t path_f32;          /* SpMV pipeline an SpMV runs per precision (cfd_spmv_path; TIMED until timed) */
+  int32_t path_f32;          /* SpMV pipeline per precision (cfd_spmv_path; TIMED until timed); with AUTO set, the
+                                pipeline it stands for, in whose place a small operator runs the direct kernel */
   int32_t path_f64;
   int32_t sliced;            /* the sliced layout (CFD_PATH_SLICED) is built */
   int32_t diagonals;         /* stored diagonals of the diagonal layout (CFD_PATH_DIAGONAL), 0 when none */
@@ -139,9 +140,13 @@ cfd_status cfd_csr_layout(const cfd_csr* a, cfd_layout_info* out);
  * it beats the record and x-staged pipelines in both precisions); otherwise
  * RECORD for FP32 (SLICED runs the plain SpMV as fast and the fused epilogues
  * slower), X_STAGED for FP64 when eligible with one thread per row, SPLIT
- * otherwise. TIMED: at the
+ * otherwise. In place of all but DIAGONAL, AUTO runs a direct kernel (every row
+ * read from global memory, nothing staged) on operators of at most 16 MB of values
+ * and columns whose longest row has at most 48 entries a thread; it has no value of
+ * its own, a set pipeline is always the one that runs. TIMED: at the
  * next SpMV in that precision, time the eligible pipelines (allocates scratch
- * vectors) and keep the fastest. */
+ * vectors), the direct kernel too where AUTO would run it, and keep the fastest
+ * (AUTO where that is the direct kernel). */
 typedef enum {
   CFD_PATH_TIMED = -2,
   CFD_PATH_AUTO = -1,
