@@ -26,7 +26,7 @@ EXPORTS = [
     "cfd_spmv", "cfd_spmv_f32",
     "cfd_amg_config_default", "cfd_amg_setup", "cfd_amg_recompute", "cfd_amg_apply", "cfd_amg_stats",
     "cfd_amg_level", "cfd_amg_set_path", "cfd_amg_destroy", "cfd_amg_setup_host", "cfd_selftest_wait_timeout",
-    "cfd_saddle_setup", "cfd_simple_apply", "cfd_block_diagonal_apply", "cfd_simple_apply_host",
+    "cfd_selftest_grid_wait_timeout", "cfd_saddle_setup", "cfd_simple_apply", "cfd_block_diagonal_apply", "cfd_simple_apply_host",
     "cfd_block_diagonal_host", "cfd_component_block_setup", "cfd_component_block_apply",
     "cfd_darcy2d_assemble", "cfd_darcy2d_theta_grad", "cfd_context_set_cluster_solve", "cfd_adjoint",
     "cfd_solve_options_default", "cfd_solve", "cfd_last_kernel_stats",
@@ -146,6 +146,7 @@ def load():
         "cfd_amg_level": (C.c_int, [P, C.c_int, C.c_int, P, P, P, P, P, P]),
         "cfd_amg_setup_host": (C.c_int, [C.c_int64, P, P, P, P, PP]),
         "cfd_selftest_wait_timeout": (C.c_int, [P, C.c_int32]),
+        "cfd_selftest_grid_wait_timeout": (C.c_int, [P, C.c_int32]),
         "cfd_amg_set_path": (C.c_int, [P, I32, I32]),
         "cfd_amg_destroy": (C.c_int, [P]),
         "cfd_solve_options_default": (None, [P]),

@@ -298,7 +298,7 @@ cfd_status check_device_flag(cfd_context* ctx) {
     cudaStreamSynchronize(ctx->stream);
     *ctx->h_err = 0;
     set_error(code == 2 ? "device-side layout check failed (int32 block in a codes-only SpMV); results are invalid"
-                               : "a device-side bounded wait ran out (bulk-copy pipeline); results are invalid");
+                               : "a device-side bounded wait ran out; results are invalid");
     return CFD_ERR_TIMEOUT;
   }
   return CFD_OK;

@@ -36,6 +36,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <mutex>
+#include <vector>
 
 #include "internal.h"
 #include "kernels.cuh"
@@ -64,6 +66,7 @@ struct GridArgs {
   DevState* st;
   int* err;
   int n, rpc, nnz_cap, far_cap, first;
+  unsigned spin;  // polls of a word before a wait gives up
 };
 
 struct GridLayout {
@@ -97,8 +100,8 @@ __device__ __forceinline__ bool gp_read(const ulonglong2* from, unsigned flag, d
   return (unsigned)(a >> 32) == flag && (unsigned)(b >> 32) == flag;
 }
 // Polls until the flag is there; false when the wait runs out.
-__device__ __forceinline__ bool gp_wait(const ulonglong2* from, unsigned flag, double& v) {
-  for (unsigned tries = 0; tries < kGpSpin; ++tries)
+__device__ __forceinline__ bool gp_wait(const ulonglong2* from, unsigned flag, double& v, unsigned spin) {
+  for (unsigned tries = 0; tries < spin; ++tries)
     if (gp_read(from, flag, v)) return true;
   return false;
 }
@@ -260,8 +263,8 @@ __global__ void __launch_bounds__(kGpThreads, 1) k_grid_pcg(GridArgs A) {
     double va = 0.0, vb = 0.0;
     int bad = 0;
     if (tid < ncta) {
-      bad = !gp_wait(sums + 2 * tid, epoch, va);
-      if (two && !bad) bad = !gp_wait(sums + 2 * tid + 1, epoch, vb);
+      bad = !gp_wait(sums + 2 * tid, epoch, va, A.spin);
+      if (two && !bad) bad = !gp_wait(sums + 2 * tid + 1, epoch, vb, A.spin);
       if (bad) atomicExch(A.err, 1);
     }
     if (warp < kGpMaxGrid / 32) {
@@ -328,7 +331,7 @@ __global__ void __launch_bounds__(kGpThreads, 1) k_grid_pcg(GridArgs A) {
     }
     for (int f = tid; f < nfar; f += kGpThreads) {
       double zf;
-      if (!gp_wait(A.z + sfar[f], (unsigned)iter + 1u, zf)) bad = 1;
+      if (!gp_wait(A.z + sfar[f], (unsigned)iter + 1u, zf, A.spin)) bad = 1;
       sp[nrow + f] = fma(beta, sp[nrow + f], zf);
     }
     if (bad) atomicExch(A.err, 1);
@@ -470,7 +473,7 @@ cfd_status grid_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, cons
   if (L.bytes > budget) return CFD_OK;
   const int rows = (rpc + kGpThreads - 1) / kGpThreads;
   GridArgs A{m.rp, m.col, m.v64, jinv, b, x, nullptr, nullptr, nullptr, nullptr, st, ctx->err, (int)n, rpc,
-             (int)nnz_cap, far_cap, 1};
+             (int)nnz_cap, far_cap, 1, kGpSpin};
   bool fits = false;
   CFD_TRY(gp_launch_rows(ctx, A, rows, grid, L.bytes, true, &fits));
   if (!fits) return CFD_OK;
@@ -512,3 +515,65 @@ cfd_status grid_pcg_solve(cfd_context* ctx, cfd_csr* a, const double* jinv, cons
 }
 
 }  // namespace cfd
+
+// The grid CG's own wait on a flag that nothing sets: a launch that goes on from a
+// state whose directions were never published, with a small bound.
+cfd_status cfd_selftest_grid_wait_timeout(cfd_context* ctx, int32_t tries) {
+  using namespace cfd;
+  if (!ctx || tries < 1) {
+    set_error("cfd_selftest_grid_wait_timeout: null context or tries < 1");
+    return CFD_ERR_CONFIG;
+  }
+  return guarded("cfd_selftest_grid_wait_timeout", [&]() -> cfd_status {
+    std::lock_guard<std::mutex> g(ctx->mu);
+    CFD_TRY_CUDA(cudaSetDevice(ctx->device));
+    const int grid = std::min(ctx->num_sms, kGpMaxGrid), rpc = 4, n = rpc * grid, nnz = 3 * n - 2;
+    std::vector<int> rp(n + 1, 0), col;
+    for (int i = 0; i < n; ++i) {
+      for (int j = std::max(0, i - 1); j <= std::min(n - 1, i + 1); ++j) col.push_back(j);
+      rp[i + 1] = (int)col.size();
+    }
+    // zeroed: vectors and values, published words (no flag set), the state (not done, iteration 0)
+    const size_t words = 4 * (size_t)kGpMaxGrid + (size_t)n;
+    const size_t bytes = words * sizeof(ulonglong2) + ((size_t)nnz + 5 * (size_t)n) * sizeof(double) + sizeof(DevState);
+    char* ws = nullptr;
+    int *drp = nullptr, *dcol = nullptr;
+    auto run = [&]() -> cfd_status {
+      CFD_TRY_CUDA(cudaMalloc((void**)&ws, bytes));
+      CFD_TRY_CUDA(cudaMalloc((void**)&drp, rp.size() * sizeof(int)));
+      CFD_TRY_CUDA(cudaMalloc((void**)&dcol, col.size() * sizeof(int)));
+      CFD_TRY_CUDA(cudaMemsetAsync(ws, 0, bytes, ctx->stream));
+      CFD_TRY_CUDA(cudaMemcpyAsync(drp, rp.data(), rp.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+      CFD_TRY_CUDA(cudaMemcpyAsync(dcol, col.data(), col.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+      GridArgs A{};
+      A.sums = reinterpret_cast<ulonglong2*>(ws);
+      A.z = A.sums + 4 * (size_t)kGpMaxGrid;
+      double* v = reinterpret_cast<double*>(ws + words * sizeof(ulonglong2));
+      A.val = v;
+      A.b = v + nnz;
+      A.x = v + nnz + n;
+      A.r = v + nnz + 2 * n;
+      A.p = v + nnz + 3 * n;
+      A.st = reinterpret_cast<DevState*>(v + nnz + 5 * (size_t)n);
+      A.rp = drp;
+      A.col = dcol;
+      A.err = ctx->err;
+      A.n = n;
+      A.rpc = rpc;
+      A.nnz_cap = 3 * rpc;
+      A.far_cap = 2;
+      A.first = 0;
+      A.spin = (unsigned)tries;
+      const GridLayout L = grid_layout(rpc, A.nnz_cap, A.far_cap);
+      bool fits = false;
+      CFD_TRY(gp_launch_rows(ctx, A, 1, grid, L.bytes, true, &fits));
+      CFD_TRY(gp_launch_rows(ctx, A, 1, grid, L.bytes, false, &fits));
+      return check_device_flag(ctx);
+    };
+    const cfd_status s = run();
+    cudaFree(ws);
+    cudaFree(drp);
+    cudaFree(dcol);
+    return s;
+  });
+}

@@ -552,6 +552,9 @@ cfd_status cfd_network_assemble_host(int32_t num_systems, const int64_t* node_of
  * by `tries`, so the path can be exercised without a fault or a hang. Returns
  * CFD_ERR_TIMEOUT with the wait's message; the context stays usable. */
 cfd_status cfd_selftest_wait_timeout(cfd_context* ctx, int32_t tries);
+/* The same for the grid CG: its kernel, polls bounded by `tries`, on directions
+ * that no CTA has published. */
+cfd_status cfd_selftest_grid_wait_timeout(cfd_context* ctx, int32_t tries);
 
 /* ---- residual without device allocation ---------------------------------
  * No counterpart in the reference: an addition for callers that cannot
