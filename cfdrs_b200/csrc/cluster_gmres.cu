@@ -13,7 +13,7 @@
 // cluster barrier (450 cycles with release and acquire), shared-memory matrix
 // reads made before that barrier, and one gather from the owner's shared memory
 // (325 cycles when remote). Measured, GMRES(30) with the pressure AMG to 1e-10:
-// 47 x 35 cells 17.5 -> 2.76 ms, 101 x 98 cells 58.8 -> 12.4 ms.
+// 47 x 35 cells 18.0 -> 2.8 ms, 101 x 98 cells 65 -> 13 ms.
 //
 // Layout: the rows of every level are split over the CTAs in equal blocks. A
 // CTA keeps its rows of A, R and P (values, columns as owner << 12 | index) and

@@ -82,8 +82,11 @@ cfd_status cfd_context_set_stream(cfd_context* ctx, void* cuda_stream);
  * (enable != 0, the default); larger ones whose rows fit the registers and shared
  * memory of the device run as one cooperative launch, FP64 GMRES (plain, Jacobi or
  * AMG) of a system that fits a cluster as one launch, and other GMRES
- * solves of up to 16 384 rows form each Arnoldi step in one cluster launch. 0
- * keeps the multi-kernel solve for every size. Same recurrence and termination; the dot products sum in another order. */
+ * solves of up to 16 384 rows form each Arnoldi step in one cluster launch. A
+ * system that fits a cluster but whose columns are scattered over its CTAs takes
+ * the cooperative launch (CG) or the multi-kernel solve (GMRES without AMG)
+ * instead, being faster there. 0 keeps the multi-kernel solve for every size. Same
+ * recurrence and termination; the dot products sum in another order. */
 cfd_status cfd_context_set_cluster_solve(cfd_context* ctx, int32_t enable);
 cfd_status cfd_context_synchronize(cfd_context* ctx);
 cfd_status cfd_context_destroy(cfd_context* ctx);

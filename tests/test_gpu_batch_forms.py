@@ -6,20 +6,18 @@ a thread; the kernels' names tell which ran."""
 import numpy as np
 import pytest
 
+from kernel_names import kernel_names
+
 pytestmark = pytest.mark.gpu
 
 
 def solve(torch, cf, systems, keep, threads, groups, prec):
-    from torch.profiler import ProfilerActivity, profile
-
     from cfdrs_b200.batch import NetworkBatch
     cfg = cf.IterativeSolverConfig(0.0, 1e-10, 20000)
     nb = NetworkBatch([A for A, _ in systems])
     nb.set_config([threads] * 4, [groups] * 4, prec)
     b = np.concatenate([q for _, q in systems])
-    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
-        x, rep = nb.solve(b, config=cfg, precision=prec)
-    names = " ".join(e.key for e in p.key_averages())
+    names, (x, rep) = kernel_names(torch, lambda: nb.solve(b, config=cfg, precision=prec))
     return x[:nb.sys_row[keep]], rep.iterations[:keep], rep.termination[:keep], names
 
 

@@ -3,17 +3,17 @@ too, and may keep it."""
 import numpy as np
 import pytest
 
+from kernel_names import kernel_names
 from test_gpu_direct_spmv import random_csr
 
 pytestmark = pytest.mark.gpu
 
 
 def kernels(torch, d, x, y, fp32):
-    from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
+    def call():
         d.spmv(x.data_ptr(), y.data_ptr(), fp32=fp32)
         d.ctx.synchronize()
-    return " ".join(e.key for e in p.key_averages())
+    return kernel_names(torch, call)[0]
 
 
 @pytest.mark.parametrize("fp32", [False, True])
