@@ -95,4 +95,6 @@ struct cfd_batch {
   std::vector<int> ls_plan_core;
   std::vector<cfd::LsPlanHead> ls_plan_host;
   std::vector<uint16_t> ls_plan_slots;
+  std::vector<int> ls_plan_rp, ls_plan_col;  // the pattern on the host, while systems are left to look at
+  int ls_plan_seen = 0;
 };

@@ -28,6 +28,19 @@ class Lists {
       if (q->node == node) return q;
     return nullptr;
   }
+  // i and j neighbours of each other, no slots yet.
+  void join(int i, int j) {
+    const int a = w_.len[i], b = w_.len[j];
+    push(i, {j, kNone, kNone, b});
+    push(j, {i, kNone, kNone, a});
+  }
+  // Drops the dead nodes of list i, the order of the others kept.
+  void compact(int i) {
+    Nb* e = std::remove_if(begin(i), end(i), [&](const Nb& q) { return !w_.alive[q.node]; });
+    w_.len[i] = (int)(e - begin(i));
+  }
+
+ private:
   void push(int i, const Nb& b) {
     if (w_.len[i] == w_.room[i]) {
       const int room = w_.room[i] ? 2 * w_.room[i] : 4;
@@ -39,13 +52,6 @@ class Lists {
     }
     begin(i)[w_.len[i]++] = b;
   }
-  void drop(int i, int node) {  // keeps the order of the others
-    Nb* q = find(i, node);
-    std::copy(q + 1, end(i), q);
-    --w_.len[i];
-  }
-
- private:
   LsPlanWork& w_;
 };
 
@@ -61,42 +67,48 @@ bool ls_plan_build(int n, const int* rp, const int* col, LsPlanWork& work, LsPla
   auto& diag = work.diag;
   diag.assign(n, kNone);
   Lists adj(work, n, nnz);
-  for (int i = 0; i < n; ++i)
+  // place[j]: where j stands in the list of the row at hand
+  auto& place = work.place;
+  place.assign(n, kNone);
+  for (int i = 0; i < n; ++i) {
+    for (int k = 0; k < adj.size(i); ++k) place[adj.begin(i)[k].node] = k;
     for (int e = rp[i]; e < rp[i + 1]; ++e) {
       const int j = col[e];
       int* s = &diag[i];
       if (j != i) {
-        Nb* q = adj.find(i, j);
-        if (!q) {
-          adj.push(j, {i, kNone, kNone});
-          adj.push(i, {j, kNone, kNone});
-          q = adj.end(i) - 1;
+        if (place[j] == kNone) {
+          place[j] = adj.size(i);
+          adj.join(i, j);
         }
-        s = &q->out;
+        s = &adj.begin(i)[place[j]].out;
       }
       if (*s == kNone) {  // a repeated entry adds into the first one's slot
         *s = slots++;
-        if (j != i) adj.find(j, i)->in = *s;
+        if (j != i) adj.begin(j)[adj.begin(i)[place[j]].rev].in = *s;
       }
       init[e - k0] = (uint16_t)*s;
     }
-  auto fill = [&](int i, int j) -> int {  // slot (i, j), the pair made where the pattern lacks it
-    Nb* q = adj.find(i, j);
-    if (q && q->out != kNone && q->in != kNone) return q->out;
-    if (!q) {
-      adj.push(i, {j, kNone, kNone});
-      adj.push(j, {i, kNone, kNone});
-      q = adj.find(i, j);
-    }
-    Nb* r = adj.find(j, i);
-    if (q->out == kNone) q->out = r->in = slots++;
-    if (q->in == kNone) q->in = r->out = slots++;
-    return q->out;
-  };
+    for (Nb* q = adj.begin(i); q != adj.end(i); ++q) place[q->node] = kNone;
+  }
+  // the pattern closed under transposition, every diagonal entry there
   for (int i = 0; i < n; ++i) {
     if (diag[i] == kNone) diag[i] = slots++;
-    for (int q = 0; q < adj.size(i); ++q) fill(i, adj.begin(i)[q].node);
+    for (Nb* q = adj.begin(i); q != adj.end(i); ++q) {
+      Nb& r = adj.begin(q->node)[q->rev];
+      if (q->out == kNone) q->out = r.in = slots++;
+      if (q->in == kNone) q->in = r.out = slots++;
+    }
   }
+  // Slot (i, j), the pair made where it is missing; looked for in the shorter list.
+  auto fill = [&](int i, int j) -> int {
+    const bool swap = adj.size(j) < adj.size(i);
+    if (const Nb* q = swap ? adj.find(j, i) : adj.find(i, j)) return swap ? q->in : q->out;
+    adj.join(i, j);
+    Nb &q = adj.end(i)[-1], &r = adj.end(j)[-1];
+    q.out = r.in = slots++;
+    q.in = r.out = slots++;
+    return q.out;
+  };
   // Right-hand-side slots are numbered after the fill: bslot(i) = ~i until then.
   auto bslot = [](int i) { return ~i; };
   auto& div = work.div;
@@ -106,6 +118,7 @@ bool ls_plan_build(int n, const int* rp, const int* col, LsPlanWork& work, LsPla
   auto& nb_end = work.nb_end;
   auto& rounds = work.rounds;
   auto& alive = work.alive;
+  auto& thin = work.thin;
   div.clear();
   upd.clear();
   nodes.clear();
@@ -114,6 +127,7 @@ bool ls_plan_build(int n, const int* rp, const int* col, LsPlanWork& work, LsPla
   rounds.clear();
   live.resize(n);
   for (int i = 0; i < n; ++i) live[i] = i;
+  constexpr int kSeen = -2;
   blocked.assign(n, -1);
   alive.assign(n, 1);
   for (int r = 0; !live.empty(); ++r) {
@@ -146,10 +160,14 @@ bool ls_plan_build(int n, const int* rp, const int* col, LsPlanWork& work, LsPla
           upd.push_back({a == c ? diag[u.node] : fill(u.node, nbs[c].node), u.in, nbs[c].out, kNone});
       }
     }
-    for (size_t q = R.node, a = R.nb; q < nodes.size(); ++q) {
-      for (; a < nb_end[q]; ++a) adj.drop(nbs[a].node, nodes[q]);
-      alive[nodes[q]] = 0;
-    }
+    for (size_t q = R.node; q < nodes.size(); ++q) alive[nodes[q]] = 0;
+    thin.clear();
+    for (size_t a = R.nb; a < nbs.size(); ++a)
+      if (blocked[nbs[a].node] == r) {  // a neighbour, not yet looked at
+        blocked[nbs[a].node] = kSeen;
+        thin.push_back(nbs[a].node);
+      }
+    for (int v : thin) adj.compact(v);
     live.erase(std::remove_if(live.begin(), live.end(), [&](int v) { return !alive[v]; }), live.end());
     rounds.push_back(R);
     if (slots + n > kLsPlanMaxSlots) return false;
@@ -231,9 +249,7 @@ bool ls_plan_build(int n, const int* rp, const int* col, LsPlanWork& work, LsPla
     }
     set.rounds.push_back(d);
   }
-  auto& place = work.place;
-  place.assign(n, kNone);
-  int core = 0;
+  int core = 0;  // place: the core's numbering from here on
   head.at_core = (int32_t)(w.size() - w0);
   for (int i : live) {
     place[i] = core++;

@@ -52,8 +52,8 @@ struct LsPlanSet {
 // Scratch of ls_plan_build, kept from one system to the next: with arrays of their
 // own for every system the builder spent half its time in the allocator.
 struct LsPlanWork {
-  struct Nb {  // a neighbour: its node, the slots of the entries to and from it
-    int node, out, in;
+  struct Nb {  // a neighbour: its node, the slots of the entries to and from it, and, while
+    int node, out, in, rev;  // lists only grow, this node's place in the neighbour's list
   };
   struct Update {  // v[target] -= v[i] v[j]; next: the target's next update of its round, -1 the last
     int target, i, j, next;
@@ -64,7 +64,7 @@ struct LsPlanWork {
   std::vector<Nb> pool;  // neighbour lists in one array
   std::vector<size_t> at;
   std::vector<int> len, room;
-  std::vector<int> diag, live, blocked, by_degree[kLsPlanDegree + 1], nodes, first, last, order, place;
+  std::vector<int> diag, live, blocked, by_degree[kLsPlanDegree + 1], nodes, first, last, order, place, thin;
   std::vector<char> alive;
   std::vector<std::pair<int, int>> div;
   std::vector<Update> upd;

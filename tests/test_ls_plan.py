@@ -186,3 +186,21 @@ def test_one_set(lib):
         np.testing.assert_array_equal(rounds[h.round0:h.round0 + h.rounds], ar)
         assert [getattr(h, f) for f in ("slots", "b0", "core", "at_core", "entries", "at_entries")] == \
             [getattr(a, f) for f in ("slots", "b0", "core", "at_core", "entries", "at_entries")]
+
+
+def test_a_hub_costs_no_more_than_a_tree(lib):
+    """A node with all others for neighbours: the builder must not search its list for
+    every one of them (a manifold of 2000 pipes took 12 times a random tree's time)."""
+    import time
+    rng = np.random.default_rng(3)
+    best = {}
+    for kind in ("star", "tree"):
+        rp, col = pattern(kind, 2000, rng)
+        times = []
+        for _ in range(7):
+            lib.clear()
+            t = time.perf_counter()
+            build(lib, 2000, rp, col)
+            times.append(time.perf_counter() - t)
+        best[kind] = min(times)
+    assert best["star"] <= 4 * best["tree"]
