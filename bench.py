@@ -671,9 +671,9 @@ def run_plain(args, world, rank, local):
 
 def run_batch(args, world, rank, local):
     """GPU arm of c4: the 1-D solve of all networks in one batched call per
-    step (cfd_batch_linear_system_solve: detection, equilibration, dense LU
-    for n <= 256, persistent CTA-per-system CG / BiCGSTAB, recheck, dense LU
-    fallback), FP64; value = the call's device time (events around copies in,
+    step (cfd_batch_linear_system_solve: detection, equilibration, direct
+    solves for n <= 256, persistent CTA-per-system CG / BiCGSTAB, recheck, direct
+    fallback, along sparse elimination plans made in the warm-up), FP64; value = the call's device time (events around copies in,
     kernels, copies out), e2e = host wall clock around the call; Jacobi-PCG per
     network (cfd_batch_solve, CUDA graph) and FP32 + refinement beside it; the
     oracle beside it on rank 0 (every BATCH_CPU_STRIDE-th network)."""
@@ -737,9 +737,9 @@ def run_batch(args, world, rank, local):
                                           + (1 if paths.get("krylov_fallback", 0) else 0)),
             "roofline": {"bound": "latency", "achieved": None, "peak": measured_peak()[0], "unit": "GB/s",
                          "frac": None, "traffic": None,
-                         "kernel": "batched 1-D solve: each Krylov system lives in shared memory for its whole "
-                                   "solve (an iteration is bound by CTA barrier latency, not HBM); the dense LU "
-                                   "fallback is FP64-FMA bound"},
+                         "kernel": "batched 1-D solve: each Krylov system lives in registers and shared memory for "
+                                   "its whole solve (an iteration is bound by shared-memory loads and reductions, "
+                                   "not HBM); the direct solves run sparse elimination plans"},
             "paths": paths, "total_iterations": rep.total_iterations, "max_iterations": rep.max_iterations,
             "max_residual": rep.max_residual,
             "fp32_refine_ms": rep32.device_ms,
