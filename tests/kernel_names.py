@@ -1,10 +1,10 @@
-"""Names of the kernels that a call launches, as torch's profiler reports them. A
-profiling session of a few microseconds, the process's first above all, may come back
-without any kernel: it is taken again."""
-import pytest
+"""Names of the kernels that a call launches, as torch's profiler reports them."""
 
 
 def kernel_names(torch, call):
+    """(names, what the call returned); names is None where the profiler reports no
+    kernel at all: a session of a few microseconds may come back empty, and in a
+    process of many contexts all of them may."""
     from torch.profiler import ProfilerActivity, profile
     for _ in range(10):
         with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
@@ -13,4 +13,4 @@ def kernel_names(torch, call):
         names = " ".join(e.key for e in p.key_averages())
         if "cfd::" in names:
             return names, out
-    pytest.skip("the profiler reports no kernels in this process")
+    return None, out
