@@ -274,7 +274,7 @@ cfd_status component_apply_device(cfd_csr* a, const T* r, T* z, const int* skip,
     gp = C->gp32;
   }
   const CbInverses I{{C->inv[0], C->inv[1], C->inv[2]}};
-  const bool wide = dense_wide(3 * (int64_t)cs);
+  const bool wide = dense_wide(3 * (int64_t)cs, false);
   const auto gemv = wide ? k_cb_gemv<4, T> : k_cb_gemv<2, T>;
   const dim3 gg((unsigned)dense_grid(cs, wide ? 4 : 2), 3);
   gemv<<<gg, kThreads, 0, s>>>(cs, I, r, z, 0, skip);

@@ -1098,13 +1098,21 @@ struct DiaVecN<float, 2> {
 // What bounds it: the matrix (33 MB for 2876 FP32 rows) comes from L2, so enough
 // of it has to be in flight: a row is shared by W warps, each lane with four 16-byte
 // loads of it and the vector's matching ones, where rows and vector start on 16-byte
-// boundaries (an n divisible by the vector); scalar loads otherwise. W is 4 while
-// all rows' warps are resident at once and 2 beyond (dense_wide); time in us of W
-// 1 / 2 / 4, and of one warp a row with scalar loads:
-//   1402 rows FP64           11.5 / 9.4 / 7.1    10.7
-//   2876 rows FP32           10.8 / 8.8 / 11.1   11.3
-//   3 x 1210 rows FP64        7.7 / 6.4 / 9.1    11.1 (three launches)
-inline bool dense_wide(int64_t rows) { return rows <= 2048; }
+// boundaries (an n divisible by the vector); scalar loads otherwise, unrolled by
+// four for FP64 (by eight or the compiler's choice 31 and 37 us at 4095 rows, 29 by
+// four) and as the compiler does for FP32 (6001 rows 17.9 us, by four 23.7, by eight
+// 19.6). W is 4 while all rows' warps are resident at once (two rows a CTA, six CTAs
+// an SM, five for an FP32 matrix) and 2 beyond (dense_wide); time in us of W 1 / 2 / 4,
+// and of one warp a row with scalar loads:
+//   1400 rows FP64            4.7 / 3.5 / 3.4     5.1
+//   1750                      5.3 / 4.2 / 4.1     5.7
+//   1900                      5.7 / 4.7 / 5.9     6.2
+//   2048                      5.9 / 4.8 / 6.2     5.9
+//   1400 rows FP32            2.9 / 2.8 / 2.6     3.4
+//   1751                      3.3 / 3.1 / 3.6     3.4
+//   2876                      5.1 / 4.6 / 5.1     5.4
+//   3 x 1210 rows FP64        7.7 / 6.4 / 9.1    11.1 (three launches, in the solve)
+inline bool dense_wide(int64_t rows, bool fp32) { return rows <= 148 * 2 * (fp32 ? 5 : 6); }
 inline int dense_grid(int n, int w) { return (n + kThreads / 32 / w - 1) / (kThreads / 32 / w); }
 
 template <int W, typename IT, typename XT>
@@ -1147,8 +1155,10 @@ __device__ __forceinline__ int dense_row_dot(int n, const IT* __restrict__ m, co
 #pragma unroll
           for (int v = 0; v < V; ++v) s += (double)av[q][v] * (double)bv[q][v];
       }
+    } else if constexpr (sizeof(IT) == 8) {
+#pragma unroll 4
+      for (int k = t; k < n; k += T) s += (double)a[k] * (double)b[k];
     } else {
-#pragma unroll 8
       for (int k = t; k < n; k += T) s += (double)a[k] * (double)b[k];
     }
     s = warp_sum(s);

@@ -1077,7 +1077,7 @@ static cfd_status vcycle(Launcher& lc, cfd_amg* amg, size_t l, const XT* b, XT* 
   const bool coarsest = (l + 1 == amg->dev.size());
   if (coarsest) {
     if (c.coarse_solve == CFD_COARSE_DENSE && amg->coarse_inv) {
-      const bool wide = dense_wide(n);
+      const bool wide = dense_wide(n, sizeof(XT) == 4 && amg->coarse_inv32);
       const int grid = dense_grid((int)n, wide ? 4 : 2);
       if (sizeof(XT) == 4 && amg->coarse_inv32)
         lc.launch(wide ? k_dense_gemv<4, XT, float> : k_dense_gemv<2, XT, float>, grid, kThreads, 0, (int)n,
