@@ -440,10 +440,11 @@ int64_t scattered_far(const HostCsr& h, int rpc) {
     const int64_t e = std::min<int64_t>(r + rpc, h.nrows);
     int64_t far = 0;
     for (int64_t i = r; i < e; ++i) {
-      const int64_t up = i > r ? h.rp[i] - h.rp[i - 1] : 0;
-      for (int64_t k = h.rp[i]; k < h.rp[i + 1]; ++k)
+      const int64_t k0 = h.rp[i], k1 = h.rp[i + 1], up = i > r ? k0 - h.rp[i - 1] : 0;
+      if (k0 == k1 || (h.ci[k0] >= r && h.ci[k1 - 1] < e)) continue;  // columns ascend: a row of the block's own
+      for (int64_t k = k0; k < k1; ++k)
         if (h.ci[k] < r || h.ci[k] >= e)
-          far += k - h.rp[i] >= up || h.ci[k - up] + 1 != h.ci[k];
+          far += k - k0 >= up || h.ci[k - up] + 1 != h.ci[k];
     }
     cap = std::max(cap, far);
   }
